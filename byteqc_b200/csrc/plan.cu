@@ -17,7 +17,15 @@
 //   prefix   : per task, the exclusive scan of its row counts and the task's
 //              tile total;
 //   launches : one per task and precision band, a fixed grid of CTAs that
-//              strides over the task's [0, total) tiles (JKTask::ntiles_dev).
+//              strides over the task's [0, total) tiles (JKTask::ntiles_dev),
+//              dealt out costly first over side streams of the plan that fork
+//              from and join the caller's stream.  The launches only add to
+//              the outputs, so their order is free, and a small build's
+//              launches (120 for the cc-pVDZ shape of H and O, 231 for the
+//              cc-pVTZ shape) are each too small to fill the GPU and as long
+//              as one quartet's chain of loads and roots: on one stream a
+//              get_jk of one water took 3.17 ms, on eight 0.88 ms (cc-pVTZ
+//              shape, two waters: 10.2 and 2.4 ms).
 //
 // Every launch of a build has the same shape each time, so a build can be
 // captured in a CUDA graph and replayed.
@@ -25,12 +33,73 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <mutex>
+#include <utility>
 #include <vector>
 #include "bqc.h"
 
 namespace {
 
 constexpr int TILE = 16;
+
+// Side streams of a plan: as many as a process has hardware queues by default.
+constexpr int SIDE_STREAMS = 8;
+
+struct SideStreams {
+    cudaStream_t side[SIDE_STREAMS];
+    cudaEvent_t fork, join[SIDE_STREAMS];
+};
+
+// Creating the streams and events takes 0.6-1 ms, as long as the rest of a
+// small molecule's set-up: a destroyed plan's set is kept for the next plan on
+// its device, at most SETS_KEPT of them.  A set belongs to one plan at a time.
+constexpr size_t SETS_KEPT = 4;
+std::mutex g_sets_lock;
+std::vector<std::pair<int, SideStreams *>> g_sets;   // (device, idle set)
+
+void free_side(SideStreams *s) {
+    for (int n = 0; n < SIDE_STREAMS; n++) {
+        if (s->side[n]) cudaStreamDestroy(s->side[n]);
+        if (s->join[n]) cudaEventDestroy(s->join[n]);
+    }
+    if (s->fork) cudaEventDestroy(s->fork);
+    delete s;
+}
+
+SideStreams *take_side(int device) {
+    {
+        std::lock_guard<std::mutex> lock(g_sets_lock);
+        for (size_t n = 0; n < g_sets.size(); n++) {
+            if (g_sets[n].first == device) {
+                SideStreams *s = g_sets[n].second;
+                g_sets.erase(g_sets.begin() + n);
+                return s;
+            }
+        }
+    }
+    SideStreams *s = new SideStreams();   // value-initialised: every handle NULL
+    bool ok = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess;
+    for (int n = 0; ok && n < SIDE_STREAMS; n++)
+        ok = cudaStreamCreateWithFlags(&s->side[n], cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&s->join[n], cudaEventDisableTiming) == cudaSuccess;
+    if (!ok) {
+        free_side(s);
+        return nullptr;
+    }
+    return s;
+}
+
+void give_side(int device, SideStreams *s) {
+    if (s == nullptr) return;
+    {
+        std::lock_guard<std::mutex> lock(g_sets_lock);
+        if (g_sets.size() < SETS_KEPT) {
+            g_sets.push_back({device, s});
+            return;
+        }
+    }
+    free_side(s);
+}
 
 // density-independent description of one task for the schedule kernels
 struct SchedTask {
@@ -47,7 +116,16 @@ struct TaskHost {
     int li, lj, lk, ll;
     int max_tiles;
     int row_off, pfx_off;   // the task's rows and prefix entries in the schedule
+    int index;              // of the task in the device arrays
+    double cost;            // estimate of its work
 };
+
+// flops of the Rys quadrature of one primitive quartet of a class
+double prim_cost(int li, int lj, int lk, int ll) {
+    auto nc = [](int l) { return (l + 1) * (l + 2) / 2; };
+    const int n = (li + lj + lk + ll) / 2 + 1;
+    return n * (15. * (li + lj + 1) * (lk + ll + 1) + 3. * nc(li) * nc(lj) * nc(lk) * nc(ll)) + 30.;
+}
 
 // Largest n in [lo, hi] such that q[c] * qr >= tol for all c < n (q
 // descending): the number of leading columns that reach tol.
@@ -158,6 +236,7 @@ struct BQCPlan {
     int nsm;
     std::vector<TaskHost> tasks;
     int ntasks, nrows_all, npfx;
+    SideStreams *streams;
     // device
     SchedTask *d_tasks;
     int *d_row_task;
@@ -239,12 +318,17 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
             s.pfx_off = pfx;
             th.row_off = s.row_off;
             th.pfx_off = pfx;
+            th.index = (int)st.size();
+            th.cost = (double)th.max_tiles * t.nprim_a * t.nprim_b * prim_cost(th.li, th.lj, th.lk, th.ll);
             pfx += nrows + 1;
             for (int r = 0; r < nrows; r++) row_task.push_back((int)st.size());
             st.push_back(s);
             p->tasks.push_back(th);
         }
     }
+    // the costly class pairs first: the others fill in behind them
+    std::stable_sort(p->tasks.begin(), p->tasks.end(),
+                     [](const TaskHost &x, const TaskHost &y) { return x.cost > y.cost; });
     p->ntasks = (int)st.size();
     p->nrows_all = (int)row_task.size();
     p->npfx = pfx;
@@ -256,7 +340,8 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
               cudaMalloc(&p->d_col0, sizeof(int) * nr) == cudaSuccess &&
               cudaMalloc(&p->d_prefix, sizeof(int) * 2 * np_) == cudaSuccess &&
               cudaMalloc(&p->d_ntiles, sizeof(int) * 2 * nt) == cudaSuccess &&
-              cudaMalloc(&p->d_dm_max, sizeof(unsigned long long)) == cudaSuccess;
+              cudaMalloc(&p->d_dm_max, sizeof(unsigned long long)) == cudaSuccess &&
+              (p->streams = take_side(p->device)) != nullptr;
     if (ok && pair_mol_host) ok = cudaMalloc(&p->d_tile_mol, sizeof(int) * tile_mol.size()) == cudaSuccess;
     if (ok && p->ntasks > 0)
         ok = cudaMemcpy(p->d_tasks, st.data(), sizeof(SchedTask) * st.size(), cudaMemcpyHostToDevice) == cudaSuccess &&
@@ -278,7 +363,7 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
 
 void BQCplan_destroy(BQCPlan *p) {
     if (p == nullptr) return;
-    cudaFree(p->d_tasks);
+    cudaFree(p->d_tasks);   // waits for the plan's launches
     cudaFree(p->d_row_task);
     cudaFree(p->d_tile_q);
     cudaFree(p->d_tile_mol);
@@ -287,6 +372,7 @@ void BQCplan_destroy(BQCPlan *p) {
     cudaFree(p->d_prefix);
     cudaFree(p->d_ntiles);
     cudaFree(p->d_dm_max);
+    give_side(p->device, p->streams);
     delete p;
 }
 
@@ -340,25 +426,32 @@ int BQCbuild_jk_plan(const BQCPlan *p, const double *pair_q, const double *dm_co
     args.n_dm = n_dm;
     args.rys = bqc_rys_table();
     args.rys_lm = bqc_rys_table_lm();
-    for (int band = 0; band < (two ? 2 : 1); band++) {
-        JKArgs a = args;
-        a.tol = band == 0 ? (two ? fp32_below : tol) : tol;
-        a.tol_hi = band == 0 ? 0. : fp32_below;
-        const int *pfx = band == 0 ? pfx0 : pfx1;
-        const int *nt = band == 0 ? nt0 : nt1;
-        for (int i = 0; i < p->ntasks; i++) {
-            const TaskHost &th = p->tasks[i];
+    const SideStreams &ss = *p->streams;
+    if (cudaEventRecord(ss.fork, stream) != cudaSuccess) return 1;
+    for (int n = 0; n < SIDE_STREAMS; n++)
+        if (cudaStreamWaitEvent(ss.side[n], ss.fork, 0) != cudaSuccess) return 1;
+    int err = 0, turn = 0;
+    for (int i = 0; i < p->ntasks && !err; i++) {
+        const TaskHost &th = p->tasks[i];
+        for (int band = 0; band < (two ? 2 : 1) && !err; band++) {
+            JKArgs a = args;
+            a.tol = band == 0 ? (two ? fp32_below : tol) : tol;
+            a.tol_hi = band == 0 ? 0. : fp32_below;
             JKTask t = th.base;
-            t.tile_prefix = pfx + th.pfx_off;
+            t.tile_prefix = (band == 0 ? pfx0 : pfx1) + th.pfx_off;
             t.tile_col0 = p->d_tile_mol ? p->d_col0 + th.row_off : nullptr;
             t.ntiles = th.max_tiles;
-            t.ntiles_dev = nt + i;
+            t.ntiles_dev = (band == 0 ? nt0 : nt1) + th.index;
             t.nsm = p->nsm;
-            int err = bqc_launch_jk(th.li, th.lj, th.lk, th.ll, a, t, band == 1, stream);
-            if (err) return err;
+            err = bqc_launch_jk(th.li, th.lj, th.lk, th.ll, a, t, band == 1, ss.side[turn++ % SIDE_STREAMS]);
         }
     }
-    return 0;
+    // join, also after a failed launch: the caller's stream waits for all of them
+    for (int n = 0; n < SIDE_STREAMS; n++)
+        if ((cudaEventRecord(ss.join[n], ss.side[n]) != cudaSuccess ||
+             cudaStreamWaitEvent(stream, ss.join[n], 0) != cudaSuccess) && !err)
+            err = 1;
+    return err;
 }
 
 }  // extern "C"

@@ -386,3 +386,32 @@ def test_repeated_builds_agree(cuda):
     dk = float((vk1 - vk0).abs().max()) / float(vk0.abs().max())
     print('repeat: relative max|dJ| %.2e max|dK| %.2e' % (dj, dk))
     assert dj < 1e-13 and dk < 1e-13
+
+
+@pytest.mark.parametrize('fp32_below', [0., 1e-6])
+def test_build_is_ordered_on_the_callers_stream(cuda, fp32_below):
+    """The build's launches run on side streams: they start after what the
+    caller's stream holds before the call (here the late arrival of the
+    density) and what follows on it sees every contribution.  Bound as in
+    test_repeated_builds_agree, for two builds."""
+    import torch
+    from byteqc_b200.scf import hf
+    mol = _mol('cc-pvdz', nw=2, seed=21)
+    opt = hf._VHFOpt(mol).build()
+    dm = torch.as_tensor(_rand_dm(mol.nao, 5) * 0.1, device=cuda)[None]
+    ref = opt.jk_ao(dm, fp32_below=fp32_below)
+    torch.cuda.synchronize()
+    big = torch.ones((4096, 4096), dtype=torch.float64, device=cuda)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        late = torch.zeros_like(dm)
+        for _ in range(3):
+            big = big @ big * 1e-4           # some milliseconds of work ahead of the copy
+        late.copy_(dm)
+        vj, vk = opt.jk_ao(late, fp32_below=fp32_below)
+        late.zero_()
+        vj, vk = vj.clone(), vk.clone()
+    s.synchronize()
+    for a, b in zip((vj, vk), ref):
+        assert float((a - b).abs().max()) < 1e-13 * float(b.abs().max())
