@@ -39,7 +39,11 @@ def _class_units():
     """One wrapper translation unit per class launcher."""
     os.makedirs(BUILD, exist_ok=True)
     units = []
-    for c in classes():
+    # the longest compilations first: quartet blocks that one thread holds
+    # unrolled, above all those that split into several launches
+    nf = lambda c: (c[0] + 1) * (c[0] + 2) * (c[1] + 1) * (c[1] + 2) * \
+        (c[2] + 1) * (c[2] + 2) * (c[3] + 1) * (c[3] + 2) // 16
+    for c in sorted(classes(), key=lambda c: (nf(c) > 162, -nf(c))):
         name = 'cls_%d%d%d%d.cu' % c
         path = os.path.join(BUILD, name)
         src = ('#include "jk_kernels.cuh"\n'
@@ -92,7 +96,7 @@ def _compile(src, extra=()):
 def build(jobs=None, verbose=True):
     if shutil.which(NVCC) is None:
         raise RuntimeError('nvcc not found: the CUDA library cannot be built')
-    units = [os.path.join(CSRC, s) for s in SOURCES] + _class_units()
+    units = _class_units() + [os.path.join(CSRC, s) for s in SOURCES]
     jobs = jobs or os.cpu_count() or 4
     with cf.ThreadPoolExecutor(jobs) as ex:
         objs = list(ex.map(_compile, units))

@@ -6,12 +6,19 @@
 
 #define BQC_LMAX 3          // s, p, d, f
 #define BQC_NCART_MAX 10
+#define PAIR_REC 4
+#define PRIM_REC 3
 
 // Everything a J/K kernel launch reads.  Device pointers unless noted.
 struct JKArgs {
     const int *pair_bra;      // shell i of each pair        (bas_pair2bra)
     const int *pair_ket;      // shell j of each pair        (bas_pair2ket)
     const double *a12, *e12, *x12, *y12, *z12;  // primitive-pair data
+    // the same data as records (a plan keeps them; NULL otherwise): per pair
+    // PAIR_REC 16-byte words {shell i, shell j, ao_loc i, ao_loc j | A, A - B},
+    // per primitive pair PRIM_REC words {a12, 1 / a12 | e12, x12 | y12, z12}
+    const int4 *pair_rec;
+    const double2 *prim_rec;
     const double *bas_x, *bas_y, *bas_z;        // shell centres
     const int *ao_loc;        // Cartesian AO offsets of the sorted, decontracted basis
     const double *pair_q;     // Schwarz factor of each pair, or NULL (no screening)
@@ -47,51 +54,94 @@ static inline JKArgs jk_args_swap_eri(const JKArgs &a) {
     return s;
 }
 
-// One rectangular (or triangular, when diag) block of the quartet space.
-struct JKTask {
+// One rectangular (or triangular, when diag) block of the quartet space: one
+// class pair.
+struct JKSub {
     int a0, na;        // bra pairs [a0, a0 + na) (global pair indices)
     int b0, nb;        // ket pairs
     int pa0, pb0;      // primitive-pair offset of the first bra / ket pair
     int nprim_a, nprim_b;  // primitive pairs per bra / ket pair
     int diag;          // bra and ket lists are the same: keep a >= b only
-    int skip_lower;    // reference rule: skip global pair index a < b
-    // Optional tile pruning.  Tiles are rows x columns of 16 x 16 quartets,
+    int rows_are_b;    // tile rows run over the b list instead of the a list
+    int row0;          // first tile row of the block among the launch's rows
+    // parts a tile runs as (at least 1 each): ranges of its quartets (a power
+    // of two up to 8) and of the primitive ket pairs
+    int rparts, kparts;
+};
+
+// the same block with bra and ket exchanged (a diagonal block has identical
+// lists on both sides; the a >= b rule stays)
+__host__ __device__ inline JKSub jk_swap_sub(const JKSub &s) {
+    JKSub t = s;
+    t.a0 = s.b0; t.na = s.nb; t.b0 = s.a0; t.nb = s.na;
+    t.pa0 = s.pb0; t.pb0 = s.pa0; t.nprim_a = s.nprim_b; t.nprim_b = s.nprim_a;
+    t.rows_are_b = !s.rows_are_b;
+    return t;
+}
+
+// What one launch covers: one block, or all blocks of one class shape.
+struct JKTask {
+    JKSub sub;         // the block, when subs is NULL
+    // Tile pruning.  Tiles are rows x columns of 16 x 16 quartets,
     // rows over the a list (or the b list when rows_are_b).  With
     // tile_prefix (device, nrows + 1 entries) row r holds the columns
     // [0, tile_prefix[r+1] - tile_prefix[r]) and block x maps to the tile
     // with tile_prefix[r] <= x < tile_prefix[r+1]; without it the grid is
     // the full rectangle.
-    const int *tile_prefix;
+    const long long *tile_prefix;
     const int *tile_col0;   // optional first column of each row (batched molecules)
     int nrows;
-    int ntiles;        // number of tiles (blocks) when tile_prefix is set
-    int rows_are_b;
+    long long ntiles;  // number of tiles when tile_prefix is set
+    // All class pairs of one shape in one launch (device arrays): the rows of
+    // the blocks follow one another, row_sub is the block of every row.
+    const JKSub *subs;
+    const int *row_sub;
+    int swapped;       // read the blocks with bra and ket exchanged
+    // K block (row shell, column shell): 0 bra shell x ket shell of the launched
+    // orientation, 1 ket x bra.  Callers add the transpose, so either is right;
+    // the flag keeps the stored halves of a class the same whichever
+    // orientation its kernel runs in.
+    int k_transposed;
     // Persistent launch: when set, the tile count lives on the device (a
     // schedule computed there) and a fixed grid of CTAs strides over the
     // tiles [0, *ntiles_dev); ntiles is then only an upper bound, and the
     // grid holds at most a few CTAs per SM of the nsm SMs.
-    const int *ntiles_dev;
+    const long long *ntiles_dev;
     int nsm;
-    // parts per tile of a group-kernel launch without ntiles_dev (set by the
+    // parts per tile of a launch without ntiles_dev (set by the
     // launcher; with ntiles_dev the kernel derives it from the device count)
     int split;
 };
 
+static inline JKTask jk_swap_task(const JKTask &t) {
+    JKTask s = t;
+    s.sub = jk_swap_sub(t.sub);
+    s.swapped = !t.swapped;
+    return s;
+}
+
 // Parts a group-kernel tile is cut into: a launch with fewer than 16 tiles
 // per SM cuts each tile into 2, 4 or 8 interleaved parts (one CTA each), so
 // that small builds still fill every SM; larger ones keep one CTA per tile.
-__host__ __device__ inline int group_split(int ntiles, int nsm) {
+__host__ __device__ inline int group_split(long long ntiles, int nsm) {
     int s = 1;
-    while (s < 8 && (long long)ntiles * s < 16LL * nsm) s *= 2;
+    while (s < 8 && ntiles * s < 16LL * nsm) s *= 2;
+    return s;
+}
+
+// The same for the kernel that gives each warp a tile: parts until every SM
+// has 32 warps, at most one per step over the tile's bra pairs.
+__host__ __device__ inline int warp_split(long long ntiles, int nsm) {
+    int s = 1;
+    while (s < 8 && ntiles * s < 32LL * nsm) s *= 2;
     return s;
 }
 
 // grid of a launch over ntiles tiles of per_tile CTAs each; persistent
 // launches cap it at ctas_per_sm CTAs on each SM
-static inline int bqc_grid(const JKTask &t, int ntiles, int per_tile, int ctas_per_sm) {
-    const long long n = (long long)ntiles * per_tile;
-    if (t.ntiles_dev == nullptr) return (int)n;
-    const long long cap = (long long)t.nsm * ctas_per_sm;
+static inline int bqc_grid(const JKTask &t, long long ntiles, int per_tile, int ctas_per_sm) {
+    const long long n = ntiles * per_tile;
+    const long long cap = t.ntiles_dev == nullptr ? 0x7fffffffLL : (long long)t.nsm * ctas_per_sm;
     return (int)(n < cap ? n : cap);
 }
 
@@ -104,9 +154,11 @@ unsigned long long bqc_count_launch(int n);
 #define BQC_VARIANT_SPLIT 2
 int bqc_class_variant(int li, int lj, int lk, int ll);
 
-// device address of the Rys coefficient table on the current device (rys_table.cu)
+// device addresses of the Rys coefficient tables on the current device
+// (rys_table.cu): RYS_POLY, RYS_POLY_LM, and the Chebyshev series RYS_TABLE
 const double *bqc_rys_table();
 const double *bqc_rys_table_lm();
+const double *bqc_rys_cheb();
 
 // launchers (jk_dispatch.cu, schwarz.cu)
 int bqc_launch_jk(int li, int lj, int lk, int ll, const JKArgs &args, const JKTask &task,

@@ -179,16 +179,16 @@ int GINTbuild_jk(BasisProdCache *bpcache, double *vj, double *vk, double *dm, in
         if (ij1 <= ij0) continue;
         JKTask t;
         memset(&t, 0, sizeof(t));
-        t.a0 = bpcache->bas_pairs_locs[cp_ij_id] + ij0;
-        t.na = ij1 - ij0;
-        t.b0 = bpcache->bas_pairs_locs[cp_kl_id] + kl0;
-        t.nb = kl1 - kl0;
-        t.pa0 = bpcache->primitive_pairs_locs[cp_ij_id] + ij0 * cij->nprim_12;
-        t.pb0 = bpcache->primitive_pairs_locs[cp_kl_id] + kl0 * ckl->nprim_12;
-        t.nprim_a = cij->nprim_12;
-        t.nprim_b = ckl->nprim_12;
-        t.diag = cp_ij_id == cp_kl_id;
-        t.skip_lower = 1;
+        t.sub.a0 = bpcache->bas_pairs_locs[cp_ij_id] + ij0;
+        t.sub.na = ij1 - ij0;
+        t.sub.b0 = bpcache->bas_pairs_locs[cp_kl_id] + kl0;
+        t.sub.nb = kl1 - kl0;
+        t.sub.pa0 = bpcache->primitive_pairs_locs[cp_ij_id] + ij0 * cij->nprim_12;
+        t.sub.pb0 = bpcache->primitive_pairs_locs[cp_kl_id] + kl0 * ckl->nprim_12;
+        t.sub.nprim_a = cij->nprim_12;
+        t.sub.nprim_b = ckl->nprim_12;
+        t.sub.rparts = t.sub.kparts = 1;
+        t.sub.diag = cp_ij_id == cp_kl_id;
         int err = bqc_launch_jk(cij->l_bra, cij->l_ket, ckl->l_bra, ckl->l_ket, args, t, 0, stream);
         if (err) return err;
     }
@@ -221,14 +221,15 @@ int GINTfill_int2e(BasisProdCache *bpcache, double *eri, int nao, int *strides, 
         if (ij1 <= ij0) continue;
         JKTask t;
         memset(&t, 0, sizeof(t));
-        t.a0 = bpcache->bas_pairs_locs[cp_ij_id] + ij0;
-        t.na = ij1 - ij0;
-        t.b0 = bpcache->bas_pairs_locs[cp_kl_id] + kl0;
-        t.nb = kl1 - kl0;
-        t.pa0 = bpcache->primitive_pairs_locs[cp_ij_id] + ij0 * cij->nprim_12;
-        t.pb0 = bpcache->primitive_pairs_locs[cp_kl_id] + kl0 * ckl->nprim_12;
-        t.nprim_a = cij->nprim_12;
-        t.nprim_b = ckl->nprim_12;
+        t.sub.a0 = bpcache->bas_pairs_locs[cp_ij_id] + ij0;
+        t.sub.na = ij1 - ij0;
+        t.sub.b0 = bpcache->bas_pairs_locs[cp_kl_id] + kl0;
+        t.sub.nb = kl1 - kl0;
+        t.sub.pa0 = bpcache->primitive_pairs_locs[cp_ij_id] + ij0 * cij->nprim_12;
+        t.sub.pb0 = bpcache->primitive_pairs_locs[cp_kl_id] + kl0 * ckl->nprim_12;
+        t.sub.nprim_a = cij->nprim_12;
+        t.sub.nprim_b = ckl->nprim_12;
+        t.sub.rparts = t.sub.kparts = 1;
         int err = bqc_launch_jk(cij->l_bra, cij->l_ket, ckl->l_bra, ckl->l_ket, args, t, 0, stream);
         if (err) return err;
     }
@@ -238,8 +239,8 @@ int GINTfill_int2e(BasisProdCache *bpcache, double *eri, int nao, int *strides, 
 // Tile rows of one class-pair task: row r (16 pairs of the a list, q sorted
 // descending) keeps the columns whose first (largest) q_b satisfies
 // q_a[16 r] q_b[16 c] dm_max >= tol; on a diagonal task also c <= r.
-static int tile_rows(const double *qa, int na, const double *qb, int nb, double dm_max, double tol,
-                     int diag, std::vector<int> &prefix) {
+static long long tile_rows(const double *qa, int na, const double *qb, int nb, double dm_max, double tol,
+                     int diag, std::vector<long long> &prefix) {
     int nta = (na + 15) / 16, ntb = (nb + 15) / 16;
     prefix.push_back(0);
     int base = (int)prefix.size() - 1;
@@ -263,8 +264,8 @@ static int tile_rows(const double *qa, int na, const double *qb, int nb, double 
 // tiles hold pairs of one molecule, grouped by molecule in increasing order and
 // sorted by their first q within a molecule.  Row r may only meet the ket
 // tiles of its own molecule, [c0, c1); col0 receives c0 per row.
-static int tile_rows_mol(const double *qa, const int *ma, int na, const double *qb, const int *mb,
-                         int nb, double dm_max, double tol, int diag, std::vector<int> &prefix,
+static long long tile_rows_mol(const double *qa, const int *ma, int na, const double *qb, const int *mb,
+                         int nb, double dm_max, double tol, int diag, std::vector<long long> &prefix,
                          std::vector<int> &col0) {
     int nta = (na + 15) / 16, ntb = (nb + 15) / 16;
     prefix.push_back(0);
@@ -304,7 +305,8 @@ static int build_jk_band(const BasisProdCache *bp, JKArgs args, const double *pa
                          int only_kl, unsigned long long *count_dev, cudaStream_t stream) {
     std::vector<JKTask> tasks;
     std::vector<int> shape;   // (li, lj, lk, ll) per task
-    std::vector<int> prefix, col0;
+    std::vector<long long> prefix;
+    std::vector<int> col0;
     std::vector<size_t> prefix_off, col0_off;
     for (int cij = 0; cij < bp->ncptype; cij++) {
         const ContractionProdType *tij = bp->cptype + cij;
@@ -317,32 +319,33 @@ static int build_jk_band(const BasisProdCache *bp, JKArgs args, const double *pa
             if (tij->l_bra > BQC_LMAX || tkl->l_bra > BQC_LMAX) return 2;
             JKTask t;
             memset(&t, 0, sizeof(t));
-            t.a0 = bp->bas_pairs_locs[cij];
-            t.na = tij->npairs;
-            t.b0 = bp->bas_pairs_locs[ckl];
-            t.nb = tkl->npairs;
-            t.pa0 = bp->primitive_pairs_locs[cij];
-            t.pb0 = bp->primitive_pairs_locs[ckl];
-            t.nprim_a = tij->nprim_12;
-            t.nprim_b = tkl->nprim_12;
-            t.diag = cij == ckl;
-            t.skip_lower = 1;
+            JKSub &s = t.sub;
+            s.a0 = bp->bas_pairs_locs[cij];
+            s.na = tij->npairs;
+            s.b0 = bp->bas_pairs_locs[ckl];
+            s.nb = tkl->npairs;
+            s.pa0 = bp->primitive_pairs_locs[cij];
+            s.pb0 = bp->primitive_pairs_locs[ckl];
+            s.nprim_a = tij->nprim_12;
+            s.nprim_b = tkl->nprim_12;
+            s.rparts = s.kparts = 1;
+            s.diag = cij == ckl;
             if (pair_q_host != nullptr) {
                 size_t off = prefix.size(), coff = col0.size();
-                int n;
+                long long n;
                 if (pair_mol_host != nullptr)
-                    n = tile_rows_mol(pair_q_host + t.a0, pair_mol_host + t.a0, t.na,
-                                      pair_q_host + t.b0, pair_mol_host + t.b0, t.nb, dm_max,
-                                      args.tol, t.diag, prefix, col0);
+                    n = tile_rows_mol(pair_q_host + s.a0, pair_mol_host + s.a0, s.na,
+                                      pair_q_host + s.b0, pair_mol_host + s.b0, s.nb, dm_max,
+                                      args.tol, s.diag, prefix, col0);
                 else
-                    n = tile_rows(pair_q_host + t.a0, t.na, pair_q_host + t.b0, t.nb, dm_max,
-                                  args.tol, t.diag, prefix);
+                    n = tile_rows(pair_q_host + s.a0, s.na, pair_q_host + s.b0, s.nb, dm_max,
+                                  args.tol, s.diag, prefix);
                 if (n == 0) {
                     prefix.resize(off);
                     col0.resize(coff);
                     continue;
                 }
-                t.nrows = (t.na + 15) / 16;
+                t.nrows = (s.na + 15) / 16;
                 t.ntiles = n;
                 prefix_off.push_back(off);
                 col0_off.push_back(coff);
@@ -354,20 +357,22 @@ static int build_jk_band(const BasisProdCache *bp, JKArgs args, const double *pa
             shape.push_back(tkl->l_ket);
         }
     }
-    int *d_prefix = nullptr;
+    // one allocation: the prefixes, then the first columns
+    long long *d_prefix = nullptr;
+    int *d_col0 = nullptr;
     if (pair_q_host != nullptr && !prefix.empty()) {
-        const size_t n_all = prefix.size() + col0.size();
-        if (cudaMallocAsync((void **)&d_prefix, sizeof(int) * n_all, stream) != cudaSuccess)
+        const size_t bytes = sizeof(long long) * prefix.size();
+        if (cudaMallocAsync((void **)&d_prefix, bytes + sizeof(int) * col0.size(), stream) != cudaSuccess)
             return 1;
-        prefix.insert(prefix.end(), col0.begin(), col0.end());
-        cudaMemcpyAsync(d_prefix, prefix.data(), sizeof(int) * n_all, cudaMemcpyHostToDevice,
-                        stream);
+        d_col0 = (int *)(d_prefix + prefix.size());
+        cudaMemcpyAsync(d_prefix, prefix.data(), bytes, cudaMemcpyHostToDevice, stream);
+        if (!col0.empty())
+            cudaMemcpyAsync(d_col0, col0.data(), sizeof(int) * col0.size(), cudaMemcpyHostToDevice, stream);
     }
-    const size_t col0_base = prefix.size() - col0.size();
     int err = 0;
     for (size_t i = 0; i < tasks.size() && !err; i++) {
         if (d_prefix) tasks[i].tile_prefix = d_prefix + prefix_off[i];
-        if (d_prefix && pair_mol_host != nullptr) tasks[i].tile_col0 = d_prefix + col0_base + col0_off[i];
+        if (d_prefix && pair_mol_host != nullptr) tasks[i].tile_col0 = d_col0 + col0_off[i];
         if (count_dev != nullptr)
             err = bqc_launch_count(args, tasks[i], count_dev, stream);
         else

@@ -3,18 +3,19 @@
 #pragma once
 #include "bqc.h"
 
-// The big coefficient table lives in one translation unit (rys_table.cu) and
-// reaches the kernels as a pointer (JKArgs::rys); the small index tables are
-// compiled into every unit.  RYS_TABLE itself is not defined here.
+// The big coefficient tables live in one translation unit (rys_table.cu) and
+// reach the kernels as pointers (JKArgs::rys, rys_lm); the small index tables are
+// compiled into every unit.  The tables themselves are not defined here.
 #define RYS_CONST_SMALL static __constant__ const
 #define RYS_NO_BIG_TABLE
 #include "rys_tables.inc"
+#include "rys_poly.inc"
 #undef RYS_NO_BIG_TABLE
 #undef RYS_CONST_SMALL
 
 namespace bqc {
 
-// number of unit intervals of the order-n table (compile-time copy of RYS_XMAX)
+// end of the order-n table (compile-time copy of RYS_XMAX)
 constexpr int kRysXmax[RYS_NMAX + 1] = {RYS_XMAX_LIST};
 
 __host__ __device__ constexpr int ncart(int l) { return (l + 1) * (l + 2) / 2; }
@@ -36,54 +37,57 @@ __host__ __device__ constexpr int cart_pow(int l, int c, int d) {
     return 0;
 }
 
+// 1/sqrt(x) of a normal positive x: the hardware's approximation refined by
+// two Newton steps y += y (1 - x y^2) / 2, each of which doubles the digits.
+// Without the special cases of rsqrt() there is no branch in the inner loop.
+__device__ __forceinline__ double rsqrt_pos(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+#pragma unroll
+    for (int n = 0; n < 2; n++) y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
+    return y;
+}
+
 // Rys nodes s = t^2 and weights of order N at x, FP64, from the fitted tables
-// (Chebyshev series on unit intervals, Gauss-Hermite limit beyond XMAX).
-// table is the level-major copy (RYS_TABLE_LM): the lanes of a warp hold
-// different x and read neighbouring addresses.
+// (polynomials on intervals of 1/RYS_PER_UNIT, Gauss-Hermite limit beyond XMAX).
+// table is the level-major copy (RYS_POLY_LM): the lanes of a warp hold
+// different x and read neighbouring addresses.  The loads bound it: 16 bytes a
+// lane are four cycles of the L1 data path at best, about eight with the
+// lanes' conflicts, against one of the FP64 pipe for the two FMAs they feed.
 template <int N>
 __device__ __forceinline__ void rys_roots(const double *__restrict__ table, double x,
                                           double *__restrict__ r, double *__restrict__ w) {
-    constexpr int nint = kRysXmax[N];
-    if (x < (double)nint) {
-        int k = (int)x;
-        double t = 2.0 * (x - k) - 1.0;
-        double t2 = t + t;
-        // level-major layout: (level kk, pair q) rows of XMAX[N] intervals
-        const double2 *c = reinterpret_cast<const double2 *>(table + RYS_TABLE_OFFSET[N]) + k;
-        double b1[2 * N], b2[2 * N];
+    constexpr int nint = RYS_PER_UNIT * kRysXmax[N];
+    const double y = RYS_PER_UNIT * x;
+    if (y < (double)nint) {
+        const int k = (int)y;
+        const double t = fma(2.0, y - k, -1.0);
+        // level-major layout: (level kk, pair q) rows of nint intervals
+        const double2 *c = reinterpret_cast<const double2 *>(table + RYS_POLY_OFFSET[N]) + k;
+        double f[2 * N];
 #pragma unroll
         for (int q = 0; q < N; q++) {
-            double2 v = __ldg(c + ((RYS_NCOEF - 1) * N + q) * nint);
-            b1[2 * q] = v.x;
-            b1[2 * q + 1] = v.y;
-            b2[2 * q] = 0.0;
-            b2[2 * q + 1] = 0.0;
+            const double2 v = __ldg(c + ((RYS_POLY_NCOEF - 1) * N + q) * nint);
+            f[2 * q] = v.x;
+            f[2 * q + 1] = v.y;
         }
 #pragma unroll
-        for (int kk = RYS_NCOEF - 2; kk >= 1; kk--) {
+        for (int kk = RYS_POLY_NCOEF - 2; kk >= 0; kk--) {
 #pragma unroll
             for (int q = 0; q < N; q++) {
-                double2 v = __ldg(c + (kk * N + q) * nint);
-                double n0 = fma(t2, b1[2 * q], v.x - b2[2 * q]);
-                double n1 = fma(t2, b1[2 * q + 1], v.y - b2[2 * q + 1]);
-                b2[2 * q] = b1[2 * q];
-                b2[2 * q + 1] = b1[2 * q + 1];
-                b1[2 * q] = n0;
-                b1[2 * q + 1] = n1;
+                const double2 v = __ldg(c + (kk * N + q) * nint);
+                f[2 * q] = fma(t, f[2 * q], v.x);
+                f[2 * q + 1] = fma(t, f[2 * q + 1], v.y);
             }
         }
+        // functions 0..N-1 are the nodes, N..2N-1 the weights
 #pragma unroll
         for (int q = 0; q < N; q++) {
-            double2 v = __ldg(c + q * nint);
-            double f0 = fma(t, b1[2 * q], v.x - b2[2 * q]);
-            double f1 = fma(t, b1[2 * q + 1], v.y - b2[2 * q + 1]);
-            // function index 2q and 2q+1: nodes are 0..N-1, weights N..2N-1
-            if (2 * q < N) r[2 * q] = f0; else w[2 * q - N] = f0;
-            if (2 * q + 1 < N) r[2 * q + 1] = f1; else w[2 * q + 1 - N] = f1;
+            r[q] = f[q];
+            w[q] = f[N + q];
         }
     } else {
-        double ix = 1.0 / x;
-        double isx = sqrt(ix);
+        const double isx = rsqrt_pos(x), ix = isx * isx;
 #pragma unroll
         for (int i = 0; i < N; i++) {
             r[i] = RYS_HERM_R2[RYS_HERM_OFFSET[N] + i] * ix;
@@ -97,23 +101,20 @@ __device__ __forceinline__ void rys_roots(const double *__restrict__ table, doub
 // same interval).
 template <int N>
 __device__ __forceinline__ double rys_one(const double *__restrict__ table, double x, int q) {
-    constexpr int nint = kRysXmax[N];
-    if (x < (double)nint) {
-        int k = (int)x;
-        double t = 2.0 * (x - k) - 1.0;
-        double t2 = t + t;
-        const double *c = table + RYS_TABLE_OFFSET[N] + k * (RYS_NCOEF * 2 * N) + q;
-        double b1 = __ldg(c + (RYS_NCOEF - 1) * 2 * N), b2 = 0.0;
+    constexpr int nint = RYS_PER_UNIT * kRysXmax[N];
+    const double y = RYS_PER_UNIT * x;
+    if (y < (double)nint) {
+        const int k = (int)y;
+        const double t = fma(2.0, y - k, -1.0);
+        const double *c = table + RYS_POLY_OFFSET[N] + k * (RYS_POLY_NCOEF * 2 * N) + q;
+        double f = __ldg(c + (RYS_POLY_NCOEF - 1) * 2 * N);
 #pragma unroll
-        for (int kk = RYS_NCOEF - 2; kk >= 1; kk--) {
-            double n0 = fma(t2, b1, __ldg(c + kk * 2 * N) - b2);
-            b2 = b1;
-            b1 = n0;
-        }
-        return fma(t, b1, __ldg(c) - b2);
+        for (int kk = RYS_POLY_NCOEF - 2; kk >= 0; kk--) f = fma(t, f, __ldg(c + kk * 2 * N));
+        return f;
     }
-    if (q < N) return RYS_HERM_R2[RYS_HERM_OFFSET[N] + q] / x;
-    return RYS_HERM_W[RYS_HERM_OFFSET[N] + q - N] * sqrt(1.0 / x);
+    const double isx = rsqrt_pos(x);
+    if (q < N) return RYS_HERM_R2[RYS_HERM_OFFSET[N] + q] * (isx * isx);
+    return RYS_HERM_W[RYS_HERM_OFFSET[N] + q - N] * isx;
 }
 
 // 2D integrals of one root and one Cartesian direction for the class

@@ -4,7 +4,7 @@
 // compile in parallel.
 #include <stdio.h>
 #include <utility>
-#include "jk_kernels.cuh"
+#include "jk_common.cuh"
 
 #define BQC_CASE(a, b, c, d) \
     int bqc_class_##a##b##c##d(const JKArgs &, const JKTask &, int, cudaStream_t);
@@ -48,13 +48,9 @@ int bqc_launch_jk(int li, int lj, int lk, int ll, const JKArgs &args, const JKTa
     JKArgs a_ = args;   // (not "a": the name is a parameter of BQC_CASE)
     if (pij < pkl) {
         a_ = jk_args_swap_eri(args);
+        t = jk_swap_task(task);
         std::swap(li, lk);
         std::swap(lj, ll);
-        t.a0 = task.b0; t.na = task.nb; t.b0 = task.a0; t.nb = task.na;
-        t.pa0 = task.pb0; t.pb0 = task.pa0; t.nprim_a = task.nprim_b; t.nprim_b = task.nprim_a;
-        t.rows_are_b = !task.rows_are_b;
-        // a bra/ket swap of a non-diagonal task changes nothing else; for a
-        // diagonal task both lists are identical and the a >= b rule is symmetric
     }
     int key = ((li * 4 + lj) * 4 + lk) * 4 + ll;
     int err = 0;
@@ -115,10 +111,11 @@ int bqc_launch_dm_cond(const double *dm, int n_dm, int nao, const int *ao_loc, i
 __global__ void count_kernel(JKArgs A, JKTask T, unsigned long long *count) {
     __shared__ int s_list[bqc::TILE * bqc::TILE];
     __shared__ int s_count;
-    const int ntiles = T.ntiles_dev != nullptr ? __ldg(T.ntiles_dev) : (int)gridDim.x;
-    for (int x = blockIdx.x; x < ntiles; x += gridDim.x) {
-        int a_begin, b_begin, n;
-        if (bqc::tile_screen(A, T, x, s_list, &s_count, a_begin, b_begin, n) && threadIdx.x == 0)
+    const long long ntiles = T.ntiles_dev != nullptr ? __ldg(T.ntiles_dev) : T.ntiles;
+    for (long long x = blockIdx.x; x < ntiles; x += gridDim.x) {
+        JKSub s;
+        int a_begin, b_begin, n, kpart;
+        if (bqc::tile_screen(A, T, x, s, s_list, &s_count, a_begin, b_begin, n, kpart) && threadIdx.x == 0)
             atomicAdd(count, (unsigned long long)n);
         __syncthreads();
     }
@@ -126,9 +123,10 @@ __global__ void count_kernel(JKArgs A, JKTask T, unsigned long long *count) {
 
 int bqc_launch_count(const JKArgs &args, const JKTask &task, unsigned long long *count,
                      cudaStream_t stream) {
-    int ntiles = task.tile_prefix ? task.ntiles : bqc::task_tiles(task);
-    if (ntiles == 0) return 0;
+    JKTask t = task;
+    t.ntiles = bqc::task_tiles(task);
+    if (t.ntiles == 0) return 0;
     bqc_count_launch(1);
-    count_kernel<<<bqc_grid(task, ntiles, 1, 8), 256, 0, stream>>>(args, task, count);
+    count_kernel<<<bqc_grid(t, t.ntiles, 1, 8), 256, 0, stream>>>(args, t, count);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }

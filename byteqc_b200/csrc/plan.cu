@@ -14,27 +14,26 @@
 //              sorted by their first q, so a binary search), at most r + 1 on
 //              a diagonal task; for batched molecules only the row's own
 //              molecule's columns count;
-//   prefix   : per task, the exclusive scan of its row counts and the task's
-//              tile total;
-//   launches : one per task and precision band, a fixed grid of CTAs that
-//              strides over the task's [0, total) tiles (JKTask::ntiles_dev),
-//              dealt out costly first over side streams of the plan that fork
-//              from and join the caller's stream.  The launches only add to
-//              the outputs, so their order is free, and a small build's
-//              launches (120 for the cc-pVDZ shape of H and O, 231 for the
-//              cc-pVTZ shape) are each too small to fill the GPU and as long
-//              as one quartet's chain of loads and roots: on one stream a
-//              get_jk of one water took 3.17 ms, on eight 0.88 ms (cc-pVTZ
-//              shape, two waters: 10.2 and 2.4 ms).
+//   prefix   : per class shape (li lj | lk ll), the exclusive scan of the row
+//              counts of all its class pairs and the shape's tile total;
+//   launches : one per shape and precision band, a fixed grid of CTAs that
+//              strides over the shape's [0, total) tiles (JKTask::ntiles_dev),
+//              spread over a few streams of the plan that fork from and join
+//              the caller's.  A basis has several groups of shells of one l
+//              (by number of primitives), so a launch per class pair would be
+//              231 launches for the cc-pVTZ shape of H and O against 55, most of
+//              them too small to fill the GPU.
 //
 // Every launch of a build has the same shape each time, so a build can be
 // captured in a CUDA graph and replayed.
 #include <algorithm>
+#include <array>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
-#include <mutex>
 #include <utility>
+#include <map>
+#include <mutex>
 #include <vector>
 #include "bqc.h"
 
@@ -101,31 +100,29 @@ void give_side(int device, SideStreams *s) {
     free_side(s);
 }
 
-// density-independent description of one task for the schedule kernels
+// density-independent description of one class pair for the schedule kernels
 struct SchedTask {
-    int row_off;   // first global row of the task (rows over the a list)
-    int nrows, ncols;
-    int a_tile0;   // first tile of the a list in the tile arrays
-    int b_tile0;
+    int row_off;   // first global row of the class pair
+    int ncols;
+    int a_tile0;   // first tile of the row list in the tile arrays
+    int b_tile0;   // of the column list
     int diag;
-    int pfx_off;   // first prefix entry of the task (nrows + 1 entries)
+    int parts;     // parts every tile runs as
 };
 
-struct TaskHost {
-    JKTask base;
+// rows [row0, row0 + nrows) of one class shape; its prefix entries start at
+// row0 + (index of the shape)
+struct SchedShape {
+    int row0, nrows;
+};
+
+struct ShapeHost {
     int li, lj, lk, ll;
-    int max_tiles;
-    int row_off, pfx_off;   // the task's rows and prefix entries in the schedule
-    int index;              // of the task in the device arrays
-    double cost;            // estimate of its work
+    int row0, nrows;
+    int index;         // in the device arrays
+    long long max_tiles;
+    double cost;
 };
-
-// flops of the Rys quadrature of one primitive quartet of a class
-double prim_cost(int li, int lj, int lk, int ll) {
-    auto nc = [](int l) { return (l + 1) * (l + 2) / 2; };
-    const int n = (li + lj + lk + ll) / 2 + 1;
-    return n * (15. * (li + lj + 1) * (lk + ll + 1) + 3. * nc(li) * nc(lj) * nc(lk) * nc(ll)) + 30.;
-}
 
 // Largest n in [lo, hi] such that q[c] * qr >= tol for all c < n (q
 // descending): the number of leading columns that reach tol.
@@ -180,51 +177,54 @@ __global__ void count_rows_kernel(const SchedTask *__restrict__ tasks, const int
     }
     const int lim = t.diag ? r - c0 + 1 : c1 - c0;
     int n0 = leading_cols(qb, c0, c1, qr, tol0) - c0;
-    cnt0[g] = max(0, min(n0, lim));
+    cnt0[g] = max(0, min(n0, lim)) * t.parts;
     if (tol1 > 0.) {
         int n1 = leading_cols(qb, c0, c1, qr, tol1) - c0;
-        cnt1[g] = max(0, min(n1, lim));
+        cnt1[g] = max(0, min(n1, lim)) * t.parts;
     }
 }
 
-// one CTA per task: exclusive scan of its row counts into the prefix and the
-// task's total
-__global__ void scan_rows_kernel(const SchedTask *__restrict__ tasks, const int *__restrict__ cnt,
-                                 int *__restrict__ prefix, int *__restrict__ ntiles) {
-    const SchedTask t = tasks[blockIdx.x];
-    __shared__ int s_warp[32];
-    __shared__ int s_carry;
+// one CTA per shape and band: exclusive scan of its row counts into the prefix
+// and the shape's total
+__global__ void scan_rows_kernel(const SchedShape *__restrict__ shapes, const int *__restrict__ cnt_all,
+                                 int cnt_stride, long long *__restrict__ prefix_all, int prefix_stride,
+                                 long long *__restrict__ ntiles_all) {
+    const SchedShape t = shapes[blockIdx.x];
+    const int *cnt = cnt_all + (size_t)blockIdx.y * cnt_stride + t.row0;
+    long long *prefix = prefix_all + (size_t)blockIdx.y * prefix_stride + t.row0 + blockIdx.x;
+    __shared__ long long s_warp[32];
+    __shared__ long long s_carry;
     if (threadIdx.x == 0) s_carry = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int base = 0; base < t.nrows; base += blockDim.x) {
         const int r = base + threadIdx.x;
-        const int v = r < t.nrows ? __ldg(cnt + t.row_off + r) : 0;
-        int x = v;   // inclusive scan within the warp
+        long long x = r < t.nrows ? __ldg(cnt + r) : 0;
+        // inclusive scan within the warp
         for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            const long long y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += y;
         }
         if (lane == 31) s_warp[warp] = x;
         __syncthreads();
         if (warp == 0) {
-            int w = lane < nw ? s_warp[lane] : 0;
+            long long w = lane < nw ? s_warp[lane] : 0;
             for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, w, o);
+                const long long y = __shfl_up_sync(0xffffffffu, w, o);
                 if (lane >= o) w += y;
             }
             if (lane < nw) s_warp[lane] = w;
         }
         __syncthreads();
-        const int incl = x + (warp > 0 ? s_warp[warp - 1] : 0) + s_carry;
-        if (r < t.nrows) prefix[t.pfx_off + r + 1] = incl;
+        const long long incl = x + (warp > 0 ? s_warp[warp - 1] : 0) + s_carry;
+        if (r < t.nrows) prefix[r + 1] = incl;
         __syncthreads();
         if (threadIdx.x == blockDim.x - 1) s_carry = incl;
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        prefix[t.pfx_off] = 0;
-        ntiles[blockIdx.x] = s_carry;
+        prefix[0] = 0;
+        ntiles_all[blockIdx.y * gridDim.x + blockIdx.x] = s_carry;
     }
 }
 
@@ -234,20 +234,74 @@ struct BQCPlan {
     const BasisProdCache *bp;
     int device;
     int nsm;
-    std::vector<TaskHost> tasks;
-    int ntasks, nrows_all, npfx;
+    std::vector<ShapeHost> shapes;   // costly first
+    int nshapes, nrows_all, npfx;
     SideStreams *streams;
     // device
     SchedTask *d_tasks;
+    SchedShape *d_shapes;
+    JKSub *d_subs;
     int *d_row_task;
     double *d_tile_q;
     int *d_tile_mol;   // NULL unless batched molecules
     int *d_cnt;        // 2 x nrows_all
     int *d_col0;       // nrows_all (batched molecules)
-    int *d_prefix;     // 2 x npfx
-    int *d_ntiles;     // 2 x ntasks
+    long long *d_prefix;   // 2 x npfx
+    long long *d_ntiles;   // 2 x nshapes
     unsigned long long *d_dm_max;
+    int4 *d_pair_rec;      // JKArgs::pair_rec, prim_rec
+    double2 *d_prim_rec;
 };
+
+namespace {
+
+// the records of JKArgs::pair_rec and prim_rec
+__global__ void pair_rec_kernel(BasisProdCache bp, int n, int4 *__restrict__ rec) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int i = bp.bas_pair2bra[t], j = bp.bas_pair2ket[t];
+    const double *x = bp.bas_coords, *y = x + bp.nbas, *z = y + bp.nbas;
+    int4 *r = rec + (size_t)t * PAIR_REC;
+    double2 *c = reinterpret_cast<double2 *>(r + 1);
+    r[0] = make_int4(i, j, bp.ao_loc[i], bp.ao_loc[j]);
+    c[0] = make_double2(x[i], y[i]);
+    c[1] = make_double2(z[i], x[i] - x[j]);
+    c[2] = make_double2(y[i] - y[j], z[i] - z[j]);
+}
+
+__global__ void prim_rec_kernel(BasisProdCache bp, int n, double2 *__restrict__ rec) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    double2 *r = rec + (size_t)t * PRIM_REC;
+    r[0] = make_double2(bp.a12[t], 1.0 / bp.a12[t]);
+    r[1] = make_double2(bp.e12[t], bp.x12[t]);
+    r[2] = make_double2(bp.y12[t], bp.z12[t]);
+}
+
+// cost of one quartet of a class shape per primitive quartet (flops of the
+// Rys quadrature), to launch the costly shapes first
+double prim_cost(int li, int lj, int lk, int ll) {
+    const int n = (li + lj + lk + ll) / 2 + 1;
+    const double nf = (li + 1) * (li + 2) / 2 * ((lj + 1) * (lj + 2) / 2) * ((lk + 1) * (lk + 2) / 2) *
+                      ((ll + 1) * (ll + 2) / 2);
+    return n * (15. * (li + lj + 1) * (lk + ll + 1) + 3. * nf) + 30.;
+}
+
+// Parts of the tiles of a class pair with many primitive quartets: a part
+// holds about PART_PRIMS primitive quartets per lane, first by fewer bra pairs
+// and then by a range of the primitives (the integrals are linear in it).  A
+// whole tile of two 6-primitive s pairs is 8 x 1296 primitive quartets in a
+// row, which no other work of a build hides.
+constexpr int PART_PRIMS = 64;
+
+void split_prims(JKSub &s) {
+    const long long n = (long long)s.nprim_a * s.nprim_b;
+    s.rparts = 1;
+    while (s.rparts < 8 && 8 / s.rparts * n > PART_PRIMS) s.rparts *= 2;
+    s.kparts = n > PART_PRIMS ? (int)((n + PART_PRIMS - 1) / PART_PRIMS) : 1;
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -278,9 +332,13 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
             if (pair_mol_host) tile_mol[class_tile0[c] + t] = pair_mol_host[p0 + t * TILE];
         }
     }
-    std::vector<SchedTask> st;
-    std::vector<int> row_task;
-    int pfx = 0;
+    // the class pairs by shape
+    struct Pair {
+        int cij, ckl;
+        JKSub sub;
+        double cost;
+    };
+    std::map<std::array<int, 4>, std::vector<Pair>> by_shape;
     for (int cij = 0; cij < bp->ncptype; cij++) {
         const ContractionProdType *tij = bp->cptype + cij;
         if (tij->npairs == 0) continue;
@@ -288,63 +346,92 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
             const ContractionProdType *tkl = bp->cptype + ckl;
             if (tkl->npairs == 0) continue;
             if (tij->l_bra > BQC_LMAX || tkl->l_bra > BQC_LMAX) { delete p; return 2; }
-            TaskHost th;
-            memset(&th, 0, sizeof(th));
-            JKTask &t = th.base;
-            t.a0 = bp->bas_pairs_locs[cij];
-            t.na = tij->npairs;
-            t.b0 = bp->bas_pairs_locs[ckl];
-            t.nb = tkl->npairs;
-            t.pa0 = bp->primitive_pairs_locs[cij];
-            t.pb0 = bp->primitive_pairs_locs[ckl];
-            t.nprim_a = tij->nprim_12;
-            t.nprim_b = tkl->nprim_12;
-            t.diag = cij == ckl;
-            t.skip_lower = 1;
-            const int nrows = (t.na + TILE - 1) / TILE, ncols = (t.nb + TILE - 1) / TILE;
-            t.nrows = nrows;
-            th.li = tij->l_bra;
-            th.lj = tij->l_ket;
-            th.lk = tkl->l_bra;
-            th.ll = tkl->l_ket;
-            th.max_tiles = t.diag ? nrows * (nrows + 1) / 2 : nrows * ncols;
-            SchedTask s;
-            s.row_off = (int)row_task.size();
-            s.nrows = nrows;
-            s.ncols = ncols;
-            s.a_tile0 = class_tile0[cij];
-            s.b_tile0 = class_tile0[ckl];
-            s.diag = t.diag;
-            s.pfx_off = pfx;
-            th.row_off = s.row_off;
-            th.pfx_off = pfx;
-            th.index = (int)st.size();
-            th.cost = (double)th.max_tiles * t.nprim_a * t.nprim_b * prim_cost(th.li, th.lj, th.lk, th.ll);
-            pfx += nrows + 1;
-            for (int r = 0; r < nrows; r++) row_task.push_back((int)st.size());
-            st.push_back(s);
-            p->tasks.push_back(th);
+            Pair x;
+            memset(&x.sub, 0, sizeof(x.sub));
+            x.cij = cij;
+            x.ckl = ckl;
+            x.sub.a0 = bp->bas_pairs_locs[cij];
+            x.sub.na = tij->npairs;
+            x.sub.b0 = bp->bas_pairs_locs[ckl];
+            x.sub.nb = tkl->npairs;
+            x.sub.pa0 = bp->primitive_pairs_locs[cij];
+            x.sub.pb0 = bp->primitive_pairs_locs[ckl];
+            x.sub.nprim_a = tij->nprim_12;
+            x.sub.nprim_b = tkl->nprim_12;
+            x.sub.diag = cij == ckl;
+            x.cost = (double)tij->nprim_12 * tkl->nprim_12;
+            split_prims(x.sub);
+            std::array<int, 4> key = {tij->l_bra, tij->l_ket, tkl->l_bra, tkl->l_ket};
+            // canonical order: pair index of the bra >= that of the ket
+            if (key[0] * (key[0] + 1) / 2 + key[1] < key[2] * (key[2] + 1) / 2 + key[3]) {
+                key = {key[2], key[3], key[0], key[1]};
+                x.sub = jk_swap_sub(x.sub);
+            }
+            by_shape[key].push_back(x);
         }
     }
-    // the costly class pairs first: the others fill in behind them
-    std::stable_sort(p->tasks.begin(), p->tasks.end(),
-                     [](const TaskHost &x, const TaskHost &y) { return x.cost > y.cost; });
-    p->ntasks = (int)st.size();
+    std::vector<SchedTask> st;
+    std::vector<SchedShape> ss;
+    std::vector<JKSub> subs;
+    std::vector<int> row_task;
+    for (auto &entry : by_shape) {
+        const std::array<int, 4> &l = entry.first;
+        // the longest quartets first: they would be the tail otherwise
+        std::stable_sort(entry.second.begin(), entry.second.end(),
+                         [](const Pair &x, const Pair &y) { return x.cost > y.cost; });
+        ShapeHost h;
+        h.li = l[0]; h.lj = l[1]; h.lk = l[2]; h.ll = l[3];
+        h.row0 = (int)row_task.size();
+        h.max_tiles = 0;
+        h.cost = 0.;
+        for (Pair &x : entry.second) {
+            const int nrows = (bp->cptype[x.cij].npairs + TILE - 1) / TILE;
+            const int ncols = (bp->cptype[x.ckl].npairs + TILE - 1) / TILE;
+            const long long tiles = x.sub.diag ? (long long)nrows * (nrows + 1) / 2 : (long long)nrows * ncols;
+            x.sub.row0 = (int)row_task.size() - h.row0;
+            SchedTask s;
+            s.row_off = (int)row_task.size();
+            s.ncols = ncols;
+            s.a_tile0 = class_tile0[x.cij];
+            s.b_tile0 = class_tile0[x.ckl];
+            s.diag = x.sub.diag;
+            s.parts = x.sub.rparts * x.sub.kparts;
+            row_task.insert(row_task.end(), nrows, (int)st.size());
+            st.push_back(s);
+            subs.push_back(x.sub);
+            h.max_tiles += tiles * s.parts;
+            h.cost += (double)tiles * x.cost * prim_cost(l[0], l[1], l[2], l[3]);
+        }
+        h.nrows = (int)row_task.size() - h.row0;
+        ss.push_back({h.row0, h.nrows});
+        p->shapes.push_back(h);
+    }
+    p->nshapes = (int)ss.size();
     p->nrows_all = (int)row_task.size();
-    p->npfx = pfx;
-    const size_t nt = std::max(p->ntasks, 1), nr = std::max(p->nrows_all, 1), np_ = std::max(pfx, 1);
+    p->npfx = p->nrows_all + p->nshapes;
+    const size_t nt = std::max<size_t>(st.size(), 1), nr = std::max(p->nrows_all, 1),
+                 np_ = std::max(p->npfx, 1), ns = std::max(p->nshapes, 1);
+    const int npair = bp->bas_pairs_locs[bp->ncptype], nprim = bp->primitive_pairs_locs[bp->ncptype];
     bool ok = cudaMalloc(&p->d_tasks, sizeof(SchedTask) * nt) == cudaSuccess &&
+              cudaMalloc(&p->d_shapes, sizeof(SchedShape) * ns) == cudaSuccess &&
+              cudaMalloc(&p->d_subs, sizeof(JKSub) * nt) == cudaSuccess &&
               cudaMalloc(&p->d_row_task, sizeof(int) * nr) == cudaSuccess &&
               cudaMalloc(&p->d_tile_q, sizeof(double) * tile_q.size()) == cudaSuccess &&
               cudaMalloc(&p->d_cnt, sizeof(int) * 2 * nr) == cudaSuccess &&
               cudaMalloc(&p->d_col0, sizeof(int) * nr) == cudaSuccess &&
-              cudaMalloc(&p->d_prefix, sizeof(int) * 2 * np_) == cudaSuccess &&
-              cudaMalloc(&p->d_ntiles, sizeof(int) * 2 * nt) == cudaSuccess &&
+              cudaMalloc(&p->d_prefix, sizeof(long long) * 2 * np_) == cudaSuccess &&
+              cudaMalloc(&p->d_ntiles, sizeof(long long) * 2 * ns) == cudaSuccess &&
               cudaMalloc(&p->d_dm_max, sizeof(unsigned long long)) == cudaSuccess &&
+              cudaMalloc(&p->d_pair_rec, sizeof(int4) * PAIR_REC * std::max(npair, 1)) == cudaSuccess &&
+              cudaMalloc(&p->d_prim_rec, sizeof(double2) * PRIM_REC * std::max(nprim, 1)) == cudaSuccess &&
               (p->streams = take_side(p->device)) != nullptr;
     if (ok && pair_mol_host) ok = cudaMalloc(&p->d_tile_mol, sizeof(int) * tile_mol.size()) == cudaSuccess;
-    if (ok && p->ntasks > 0)
+    if (ok && p->nshapes > 0)
         ok = cudaMemcpy(p->d_tasks, st.data(), sizeof(SchedTask) * st.size(), cudaMemcpyHostToDevice) == cudaSuccess &&
+             cudaMemcpy(p->d_shapes, ss.data(), sizeof(SchedShape) * ss.size(), cudaMemcpyHostToDevice) ==
+                 cudaSuccess &&
+             cudaMemcpy(p->d_subs, subs.data(), sizeof(JKSub) * subs.size(), cudaMemcpyHostToDevice) ==
+                 cudaSuccess &&
              cudaMemcpy(p->d_row_task, row_task.data(), sizeof(int) * row_task.size(),
                         cudaMemcpyHostToDevice) == cudaSuccess;
     if (ok)
@@ -353,10 +440,22 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
     if (ok && pair_mol_host)
         ok = cudaMemcpy(p->d_tile_mol, tile_mol.data(), sizeof(int) * tile_mol.size(),
                         cudaMemcpyHostToDevice) == cudaSuccess;
+    if (ok && npair > 0 && nprim > 0) {
+        // done before the plan is handed out: builds may come on any stream
+        pair_rec_kernel<<<(npair + 255) / 256, 256>>>(*bp, npair, p->d_pair_rec);
+        prim_rec_kernel<<<(nprim + 255) / 256, 256>>>(*bp, nprim, p->d_prim_rec);
+        bqc_count_launch(2);
+        ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess;
+    }
     if (!ok) {
         BQCplan_destroy(p);
         return 1;
     }
+    // costly shapes first, so that the cheap ones fill the tail
+    // (the rows and prefixes stay in the order of the device arrays)
+    for (int n = 0; n < p->nshapes; n++) p->shapes[n].index = n;
+    std::stable_sort(p->shapes.begin(), p->shapes.end(),
+                     [](const ShapeHost &x, const ShapeHost &y) { return x.cost > y.cost; });
     *out = p;
     return 0;
 }
@@ -364,6 +463,8 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
 void BQCplan_destroy(BQCPlan *p) {
     if (p == nullptr) return;
     cudaFree(p->d_tasks);   // waits for the plan's launches
+    cudaFree(p->d_shapes);
+    cudaFree(p->d_subs);
     cudaFree(p->d_row_task);
     cudaFree(p->d_tile_q);
     cudaFree(p->d_tile_mol);
@@ -372,6 +473,8 @@ void BQCplan_destroy(BQCPlan *p) {
     cudaFree(p->d_prefix);
     cudaFree(p->d_ntiles);
     cudaFree(p->d_dm_max);
+    cudaFree(p->d_pair_rec);
+    cudaFree(p->d_prim_rec);
     give_side(p->device, p->streams);
     delete p;
 }
@@ -380,7 +483,7 @@ int BQCbuild_jk_plan(const BQCPlan *p, const double *pair_q, const double *dm_co
                      double *vk, const double *dm, int nao, int n_dm, double tol, double fp32_below,
                      cudaStream_t stream) {
     if (p == nullptr || pair_q == nullptr || dm_cond == nullptr || dm == nullptr) return 3;
-    if (p->ntasks == 0) return 0;
+    if (p->nshapes == 0) return 0;
     const BasisProdCache *bp = p->bp;
     const bool two = fp32_below > tol;
     // 1. dm_max on the device
@@ -394,13 +497,9 @@ int BQCbuild_jk_plan(const BQCPlan *p, const double *pair_q, const double *dm_co
     count_rows_kernel<<<(p->nrows_all + 255) / 256, 256, 0, stream>>>(
         p->d_tasks, p->d_row_task, p->nrows_all, p->d_tile_q, p->d_tile_mol, p->d_dm_max,
         two ? fp32_below : tol, two ? tol : 0., cnt0, cnt1, p->d_col0);
-    int *pfx0 = p->d_prefix, *pfx1 = p->d_prefix + std::max(p->npfx, 1);
-    int *nt0 = p->d_ntiles, *nt1 = p->d_ntiles + std::max(p->ntasks, 1);
-    scan_rows_kernel<<<p->ntasks, 1024, 0, stream>>>(p->d_tasks, cnt0, pfx0, nt0);
-    if (two) {
-        bqc_count_launch(1);
-        scan_rows_kernel<<<p->ntasks, 1024, 0, stream>>>(p->d_tasks, cnt1, pfx1, nt1);
-    }
+    const int nr = std::max(p->nrows_all, 1), np_ = std::max(p->npfx, 1);
+    scan_rows_kernel<<<dim3(p->nshapes, two ? 2 : 1), 1024, 0, stream>>>(p->d_shapes, p->d_cnt, nr,
+                                                                         p->d_prefix, np_, p->d_ntiles);
     if (cudaGetLastError() != cudaSuccess) return 1;
     // 3. the class kernels, persistent over the device tile counts
     JKArgs args;
@@ -409,6 +508,8 @@ int BQCbuild_jk_plan(const BQCPlan *p, const double *pair_q, const double *dm_co
     args.pair_ket = bp->bas_pair2ket;
     args.a12 = bp->a12;
     args.e12 = bp->e12;
+    args.pair_rec = p->d_pair_rec;
+    args.prim_rec = p->d_prim_rec;
     args.x12 = bp->x12;
     args.y12 = bp->y12;
     args.z12 = bp->z12;
@@ -426,31 +527,36 @@ int BQCbuild_jk_plan(const BQCPlan *p, const double *pair_q, const double *dm_co
     args.n_dm = n_dm;
     args.rys = bqc_rys_table();
     args.rys_lm = bqc_rys_table_lm();
+    // fork: the shapes are independent (the outputs are accumulated by atomics)
     const SideStreams &ss = *p->streams;
     if (cudaEventRecord(ss.fork, stream) != cudaSuccess) return 1;
     for (int n = 0; n < SIDE_STREAMS; n++)
         if (cudaStreamWaitEvent(ss.side[n], ss.fork, 0) != cudaSuccess) return 1;
     int err = 0, turn = 0;
-    for (int i = 0; i < p->ntasks && !err; i++) {
-        const TaskHost &th = p->tasks[i];
+    for (int i = 0; i < p->nshapes && !err; i++) {
+        const ShapeHost &h = p->shapes[i];
         for (int band = 0; band < (two ? 2 : 1) && !err; band++) {
             JKArgs a = args;
             a.tol = band == 0 ? (two ? fp32_below : tol) : tol;
             a.tol_hi = band == 0 ? 0. : fp32_below;
-            JKTask t = th.base;
-            t.tile_prefix = (band == 0 ? pfx0 : pfx1) + th.pfx_off;
-            t.tile_col0 = p->d_tile_mol ? p->d_col0 + th.row_off : nullptr;
-            t.ntiles = th.max_tiles;
-            t.ntiles_dev = (band == 0 ? nt0 : nt1) + th.index;
+            JKTask t;
+            memset(&t, 0, sizeof(t));
+            t.tile_prefix = p->d_prefix + (size_t)band * np_ + h.row0 + h.index;
+            t.tile_col0 = p->d_tile_mol ? p->d_col0 + h.row0 : nullptr;
+            t.nrows = h.nrows;
+            t.ntiles = h.max_tiles;
+            t.subs = p->d_subs;
+            t.row_sub = p->d_row_task + h.row0;
+            t.ntiles_dev = p->d_ntiles + (size_t)band * p->nshapes + h.index;
             t.nsm = p->nsm;
-            err = bqc_launch_jk(th.li, th.lj, th.lk, th.ll, a, t, band == 1, ss.side[turn++ % SIDE_STREAMS]);
+            err = bqc_launch_jk(h.li, h.lj, h.lk, h.ll, a, t, band == 1, ss.side[turn++ % SIDE_STREAMS]);
         }
     }
-    // join, also after a failed launch: the caller's stream waits for all of them
+    // join, also after a failed launch: the caller's stream waits for all
     for (int n = 0; n < SIDE_STREAMS; n++)
-        if ((cudaEventRecord(ss.join[n], ss.side[n]) != cudaSuccess ||
-             cudaStreamWaitEvent(stream, ss.join[n], 0) != cudaSuccess) && !err)
-            err = 1;
+        if (cudaEventRecord(ss.join[n], ss.side[n]) != cudaSuccess ||
+            cudaStreamWaitEvent(stream, ss.join[n], 0) != cudaSuccess)
+            err = err ? err : 1;
     return err;
 }
 

@@ -20,13 +20,21 @@ tables are not used here.  This script derives its own from the mathematics:
 * for 0 <= x < XMAX[n] the range is cut into unit intervals and every node and
   weight is interpolated at the 12 Chebyshev points of each interval
   (degree-11 Chebyshev series, evaluated with Clenshaw's recurrence);
+* the J/K kernels use a second fit of the same functions: intervals of 1/2, the
+  interpolant at 10 Chebyshev points stored as a degree-9 polynomial in
+  t = -1 .. 1 over the interval (Horner's rule; the Chebyshev coefficients fall
+  so fast that the monomial ones do too, and the sum loses nothing).  Its
+  remainder, (1/4)^10 / (2^9 10!) = 5e-16 times a derivative, is that of the
+  unit intervals, (1/2)^12 / (2^11 12!) = 2.5e-16, with 10 coefficients to load
+  instead of 12 and 9 operations instead of 22;
 * for x >= XMAX[n] the quadrature is the half-range Gauss-Hermite rule:
   s_i = h_i^2 / x, w_i = W_i / sqrt(x), where h_i > 0 are the positive roots of
   the Hermite polynomial H_2n and W_i their Gauss-Hermite weights.  XMAX[n] is
   the first integer at which this limit agrees with the exact rule to 1e-15.
 
-Output: ``byteqc_b200/csrc/rys_tables.inc`` (C source, included by the CUDA
-library) and ``rys_tables_report.json`` (fit errors measured at off-node points).
+Output: ``byteqc_b200/csrc/rys_tables.inc`` and ``rys_poly.inc`` (C source,
+included by the CUDA library: the Chebyshev series, which the Schwarz factors
+are evaluated with, and the polynomials of the J/K kernels) and ``rys_tables_report.json`` (fit errors measured at off-node points).
 
 Run:  python -m byteqc_b200.rys.gen_rys_tables   (about a minute on 8 cores)
 """
@@ -39,10 +47,13 @@ import mpmath as mp
 
 NMAX = 7          # s-f shell quartets: L <= 12  ->  n <= 7
 DEG = 11          # Chebyshev degree per unit interval
+POLY_DEG = 9      # degree of the polynomials
+PER_UNIT = 2      # their intervals per unit of x
 DPS = 60
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 OUT_INC = os.path.join(HERE, '..', 'csrc', 'rys_tables.inc')
+OUT_POLY = os.path.join(HERE, '..', 'csrc', 'rys_poly.inc')
 OUT_REPORT = os.path.join(HERE, 'rys_tables_report.json')
 
 
@@ -111,8 +122,8 @@ def find_xmax(n, herm):
         x += 1
 
 
-def _cheb_nodes():
-    N = DEG + 1
+def _cheb_nodes(deg=DEG):
+    N = deg + 1
     return [mp.cos(mp.pi * (k + mp.mpf(1) / 2) / N) for k in range(N)]
 
 
@@ -144,6 +155,69 @@ def fit_interval(args):
     return n, a, coefs, err
 
 
+def fit_poly(args):
+    """Monomial coefficients over interval a of 1 / PER_UNIT, and the error of
+    the double-precision Horner sum off the nodes."""
+    n, a = args
+    mp.mp.dps = DPS
+    N = POLY_DEG + 1
+    vals = [rys_exact(n, (a + mp.mpf(1) / 2 + t / 2) / PER_UNIT) for t in _cheb_nodes(POLY_DEG)]
+    funcs = [[v[0][i] for v in vals] for i in range(n)] + \
+            [[v[1][i] for v in vals] for i in range(n)]
+    # monomials of the Chebyshev polynomials T_0 .. T_DEG
+    cheb = [[mp.mpf(1)], [mp.mpf(0), mp.mpf(1)]]
+    while len(cheb) < N:
+        up = [mp.mpf(0)] + [2 * c for c in cheb[-1]]
+        cheb.append([c - (cheb[-2][i] if i < len(cheb[-2]) else 0) for i, c in enumerate(up)])
+    coefs = []
+    for f in funcs:
+        c = [2 * mp.fsum(f[k] * mp.cos(mp.pi * j * (k + mp.mpf(1) / 2) / N)
+                         for k in range(N)) / N for j in range(N)]
+        c[0] /= 2
+        coefs.append([float(mp.fsum(c[j] * cheb[j][i] for j in range(i, N))) for i in range(N)])
+    err = 0.0
+    for t in (-0.93, -0.41, 0.05, 0.57, 0.96):
+        r, w = rys_exact(n, (a + mp.mpf(1) / 2 + mp.mpf(t) / 2) / PER_UNIT)
+        for exact, c in zip(r + w, coefs):
+            val = 0.0
+            for cj in reversed(c):
+                val = val * t + cj
+            err = max(err, abs(val / float(exact) - 1))
+    return n, a, coefs, err
+
+
+def write_poly(xmax, results):
+    table = {(n, a): coefs for n, a, coefs, _ in results}
+    nk = POLY_DEG + 1
+    offs = [0]
+    for n in range(1, NMAX + 1):
+        offs.append(offs[-1] + PER_UNIT * xmax[n] * nk * 2 * n)
+    lines = ['// Generated by byteqc_b200/rys/gen_rys_tables.py; do not edit.',
+             '// Rys nodes s=t^2 and weights: degree-%d polynomials in t = -1 .. 1' % POLY_DEG,
+             '// on intervals of 1/RYS_PER_UNIT of x in [0, XMAX[n]).',
+             '// Two layouts of the same coefficients, in the storage and order of',
+             '// rys_tables.inc: RYS_POLY, interval-major, per (n, interval a)',
+             '// [coef k = 0..%d][q = 0..2n-1]; RYS_POLY_LM, level-major, per n' % POLY_DEG,
+             '// [k][pair p = 0..n-1][interval a][2].',
+             '#define RYS_POLY_NCOEF %d' % nk,
+             '#define RYS_PER_UNIT %d' % PER_UNIT,
+             'RYS_CONST_SMALL int RYS_POLY_OFFSET[%d] = {0, %s};' % (NMAX + 2, ', '.join(str(o) for o in offs)),
+             '#ifndef RYS_NO_BIG_TABLE',
+             'RYS_CONST double RYS_POLY[%d] = {' % offs[-1]]
+    row = lambda vals: '  ' + ', '.join('%.17g' % v for v in vals) + ','
+    for n in range(1, NMAX + 1):
+        for a in range(PER_UNIT * xmax[n]):
+            lines.append(row(table[n, a][q][k] for k in range(nk) for q in range(2 * n)))
+    lines += ['};', 'RYS_CONST double RYS_POLY_LM[%d] = {' % offs[-1]]
+    for n in range(1, NMAX + 1):
+        for k in range(nk):
+            for p in range(n):
+                lines.append(row(table[n, a][2 * p + e][k] for a in range(PER_UNIT * xmax[n]) for e in range(2)))
+    lines += ['};', '#endif']
+    with open(OUT_POLY, 'w') as f:
+        f.write('\n'.join(lines) + '\n')
+
+
 def main():
     herm = {n: hermite_half(n) for n in range(1, NMAX + 1)}
     xmax = {n: find_xmax(n, herm[n]) for n in range(1, NMAX + 1)}
@@ -151,6 +225,8 @@ def main():
     jobs = [(n, a) for n in range(1, NMAX + 1) for a in range(xmax[n])]
     with mproc.get_context('spawn').Pool(os.cpu_count()) as pool:
         results = pool.map(fit_interval, jobs, chunksize=4)
+        poly = pool.map(fit_poly, [(n, a) for n in range(1, NMAX + 1) for a in range(PER_UNIT * xmax[n])],
+                        chunksize=4)
     table = {}
     errs = {}
     for n, a, coefs, err in results:
@@ -219,8 +295,11 @@ def main():
         '%.17g' % float(W) for n in range(1, NMAX + 1) for h, W in herm[n])))
     with open(OUT_INC, 'w') as f:
         f.write('\n'.join(lines) + '\n')
+    write_poly(xmax, poly)
+    perrs = {n: max(e for m, _, _, e in poly if m == n) for n in xmax}
     with open(OUT_REPORT, 'w') as f:
-        json.dump({'xmax': xmax, 'deg': DEG, 'max_rel_fit_error': errs}, f, indent=1)
+        json.dump({'xmax': xmax, 'deg': DEG, 'max_rel_fit_error': errs,
+                   'poly': {'deg': POLY_DEG, 'per_unit': PER_UNIT, 'max_rel_fit_error': perrs}}, f, indent=1)
 
 
 if __name__ == '__main__':

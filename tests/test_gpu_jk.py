@@ -415,3 +415,88 @@ def test_build_is_ordered_on_the_callers_stream(cuda, fp32_below):
     s.synchronize()
     for a, b in zip((vj, vk), ref):
         assert float((a - b).abs().max()) < 1e-13 * float(b.abs().max())
+
+
+@pytest.mark.parametrize('nc,n_dm,fp32_below', [(1, 1, 0.), (3, 1, 0.), (3, 2, 0.), (3, 1, 1e-6)])
+def test_primitive_parts_match_whole_tiles(cuda, nc, n_dm, fp32_below):
+    """A plan cuts the tiles of strongly contracted class pairs into ranges of
+    their primitive quartets (up to 1296 for two pairs of 6-primitive s
+    shells); the host-scheduled build runs whole tiles.  Same sums in another
+    order: the bound of test_device_schedule_matches_host_pruning."""
+    import ctypes
+    import torch
+    from byteqc_b200 import lib as L
+    from byteqc_b200.scf import hf
+    from byteqc_b200.scf.hf import _ptr, _stream
+    lib = L.load_library()
+    mol = Mole(linear_alkane(nc), synthetic_basis('6-31g**', ['C', 'H']))
+    opt = hf._VHFOpt(mol).build()
+    d = np.stack([_rand_dm(mol.nao, s) for s in range(n_dm)]) * 0.1
+    C = opt.coeff_dev
+    dmc = (C @ torch.as_tensor(d, device=cuda) @ C.T).contiguous()
+    nao = dmc.shape[-1]
+    cond = torch.empty((opt.mol.nbas, opt.mol.nbas), dtype=torch.float64, device=cuda)
+    assert lib.BQCdm_cond(_ptr(dmc), n_dm, nao, _ptr(opt._mem['ao_loc']), opt.mol.nbas, _ptr(cond),
+                          _stream()) == 0
+    out = []
+    for plan in (False, True):
+        vj, vk = torch.zeros_like(dmc), torch.zeros_like(dmc)
+        if plan:
+            err = lib.BQCbuild_jk_plan(opt._plan, _ptr(opt.pair_q), _ptr(cond), _ptr(vj), _ptr(vk),
+                                       _ptr(dmc), nao, n_dm, opt.direct_scf_tol, fp32_below, _stream())
+        else:
+            err = lib.BQCbuild_jk(ctypes.cast(opt.bpcache, ctypes.c_void_p), _ptr(opt.pair_q),
+                                  opt.pair_q_host.ctypes.data_as(ctypes.c_void_p), _ptr(cond),
+                                  float(cond.max()), _ptr(vj), _ptr(vk), _ptr(dmc), nao, n_dm,
+                                  opt.direct_scf_tol, fp32_below, None, _stream())
+        assert err == 0
+        out.append((vj, vk))
+    torch.cuda.synchronize()
+    for a, b in zip(*out):
+        assert float(a.abs().max()) > 0
+        # FP32 integrals are summed over the primitives in FP32: their order
+        # changes them by their rounding, 1e-7 of quartets below 1e-6
+        tol = 1e-12 * max(1., float(a.abs().max())) if fp32_below == 0. else 1e-10
+        assert float((a - b).abs().max()) < tol
+
+
+@pytest.mark.parametrize('kind,bra,ket', [('cc-pvdz', (2, 0), (1, 1)), ('cc-pvdz', (1, 1), (2, 2)),
+                                          ('cc-pvdz', (1, 0), (2, 2)), ('cc-pvtz', (3, 0), (1, 1)),
+                                          ('cc-pvtz', (1, 1), (3, 3)), ('cc-pvtz', (2, 0), (3, 3))])
+def test_stored_half_of_k(cuda, kind, bra, ket):
+    """V holds a class's exchange contributions with the rows at the shells of
+    its bra pair, whichever orientation the kernel runs in: (2, 2) and (3, 3)
+    pairs with a larger component count are the ket of the smaller pair in
+    the group kernel, (2, 2) pairs the bra of (1, 0) in the split launches."""
+    import ctypes
+    import torch
+    from byteqc_b200 import lib as L
+    from byteqc_b200.scf import hf
+    from byteqc_b200.scf.hf import _ptr, _stream
+    lib = L.load_library()
+    mol = _mol(kind, nw=2, seed=8)
+    opt = hf._VHFOpt(mol).build()
+    if bra == (1, 0) and ket == (2, 2):
+        bra, ket = ket, bra
+    C = opt.coeff_dev
+    dmc = (C @ torch.as_tensor(_rand_dm(mol.nao, 3), device=cuda) @ C.T)[None].contiguous()
+    nao = dmc.shape[-1]
+    l_of = np.repeat(opt.mol._bas[:, 1], (opt.mol._bas[:, 1] + 1) * (opt.mol._bas[:, 1] + 2) // 2)
+    vk = torch.zeros_like(dmc)
+    n = 0
+    for ci in range(opt.ncptype):
+        for ck in range(ci + 1):
+            a, b = opt.cptype[ci][:2], opt.cptype[ck][:2]
+            if sorted([a, b]) != sorted([bra, ket]) or not (opt.cptype[ci][3] and opt.cptype[ck][3]):
+                continue
+            assert lib.BQCbuild_jk_class(ctypes.cast(opt.bpcache, ctypes.c_void_p), ci, ck, _ptr(opt.pair_q),
+                                         opt.pair_q_host.ctypes.data_as(ctypes.c_void_p), None, 1., None,
+                                         _ptr(vk), _ptr(dmc), nao, 1, opt.direct_scf_tol ** 2, 0., None,
+                                         _stream()) == 0
+            n += 1
+    torch.cuda.synchronize()
+    K = vk[0].cpu().numpy()
+    rows = np.isin(l_of, bra)
+    cols = np.isin(l_of, ket)
+    assert n > 0 and abs(K[np.ix_(rows, cols)]).max() > 0
+    assert abs(K[~rows]).max() == 0 and abs(K[:, ~cols]).max() == 0
