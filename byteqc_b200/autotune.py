@@ -18,7 +18,7 @@ import json
 
 import numpy as np
 
-SMALL_NF = 54          # jk_kernels.cuh SMALL_NF
+SMALL_NF = 54          # jk_common.cuh SMALL_NF
 MAX_SPLIT = 3          # jk_kernels.cuh MAX_SPLIT
 GROUP, SPLIT = 1, 2    # BQC_VARIANT_GROUP, BQC_VARIANT_SPLIT
 

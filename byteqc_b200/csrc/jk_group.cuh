@@ -4,6 +4,17 @@
 
 namespace bqc {
 
+// Shared-memory traffic bounds it: the table loads of the products, the
+// density blocks and the reductions.  A thread therefore owns as many
+// components as its registers hold (at most ACC_MAX = 60): the rows of the 2D
+// tables and the density values it loads serve TJ fj at once, and fewer
+// threads meet in the reductions.  Against one (fi, fj) and at most 36
+// components a thread, one build of (H2O)_11 / cc-pVTZ on B200: (fd|dp)
+// 2.67 -> 1.70 ms, (fd|fp) 1.30 -> 0.72 ms, (ff|fp) 1.05 -> 0.38 ms, (fp|pp)
+// 2.41 -> 1.71 ms, (dp|dp) 3.30 -> 2.71 ms, (fp|dp) 2.66 -> 2.34 ms; the (fd|
+// and (ff| classes gain most, whose ket components had been dealt to two or
+// three threads that loaded all three factors of every product.
+//
 // A quartet (LI LJ | LK LL) runs on TPQ threads; thread (fi, jc, chunk) owns
 // the components (fi, fj, fk, fl) with fj in [jc TJ, (jc + 1) TJ), fk in its
 // chunk and every fl.
