@@ -1,6 +1,17 @@
 // One thread per quartet: J/K kernel of the shell-quartet classes of at most
 // SMALL_NF Cartesian components, and, as launches over ranges of the
 // components of shell k, of the classes that split into a few such ranges.
+//
+// A warp takes a 16 x 16 tile: a lane holds one ket pair and steps over the
+// bra pairs, two a step (one per half warp).  What a lane needs of its ket
+// pair is read once a tile, what belongs to a bra pair is the same address for
+// 16 lanes, and only D_jl, its bound and the atomic on K_jl are per quartet;
+// the 128-thread half tiles that this replaces read all of it per quartet
+// (77 % of the L1 wavefront peak for (ps|ss)) and met at block barriers.
+// Measured on B200, one build of (H2O)_32 / cc-pVDZ: (ps|ss) 18.7 -> 14.3 ms,
+// (ss|ss) 10.3 -> 8.0 ms, (ps|ps) 11.6 -> 8.7 ms, (ds|ds) 1.10 -> 0.74 ms, but
+// (dp|ps) 4.1 -> 4.2 ms and (ds|pp) 2.3 -> 2.6 ms.  What bounds it now is
+// latency: 0.43 instructions a cycle and scheduler at 16 warps an SM.
 #pragma once
 #include "jk_common.cuh"
 
@@ -55,12 +66,18 @@ struct WarpCfg {
     static constexpr int NF = NFI * NFJ * NFK * NFL;
     // sums carried over the bra pairs of a tile: J_kl, K_il, K_ik
     static constexpr int PERS = NFK * NFL + NFI * NFL + NFI * NFK;
-    // in registers beside the quartet block where both fit, else in shared
-    // memory, one column per lane
+    // in registers beside the quartet block where both fit (64 doubles are half
+    // of the largest register budget), else in shared memory, one column per
+    // lane, which no other lane touches
     static constexpr bool SMEM_SUMS = NF + PERS > 64;
     static constexpr int SMEM = SMEM_SUMS ? PERS * WARP_CTA * (int)sizeof(double) : 0;
-    // CTAs per SM of the register budget
-    static constexpr int MINB = NF == 1 ? 5 : (NF <= 3 ? 4 : (NF <= 9 ? 3 : 2));
+    // CTAs per SM of the register budget: 64, 128, 168 and 255 registers.  One
+    // build of (H2O)_32 / cc-pVDZ and of C60H122 / 6-31G** on B200: (ss|ss), whose
+    // block is one double, 8.0 and 9.2 ms at 96 registers, 6.7 and 7.3 ms at 64
+    // in spite of some spills; (ps|ss) 14.2 and 17.6 ms at 128, 16.5 and 21.7
+    // ms at 80; (ps|ps) 8.8 and 11.2 ms at 168, 9.3 and 11.5 ms at 128; (dp|ps)
+    // 4.2 and 7.2 ms at 255, 6.3 and 11.3 ms at 168.
+    static constexpr int MINB = NF == 1 ? 8 : (NF <= 3 ? 4 : (NF <= 9 ? 3 : 2));
 };
 
 template <int LI, int LJ, int LK, int LL, typename F, int K0 = 0, int KN = ncart(LK)>
