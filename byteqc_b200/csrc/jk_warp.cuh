@@ -9,7 +9,7 @@
 // the 128-thread half tiles that this replaces read all of it per quartet
 // (77 % of the L1 wavefront peak for (ps|ss)) and met at block barriers.
 // Measured on B200, one build of (H2O)_32 / cc-pVDZ: (ps|ss) 18.7 -> 14.3 ms,
-// (ss|ss) 10.3 -> 8.0 ms, (ps|ps) 11.6 -> 8.7 ms, (ds|ds) 1.10 -> 0.74 ms, but
+// (ss|ss) 10.3 -> 6.7 ms, (ps|ps) 11.6 -> 8.7 ms, (ds|ds) 1.10 -> 0.74 ms, but
 // (dp|ps) 4.1 -> 4.2 ms and (ds|pp) 2.3 -> 2.6 ms.  What bounds it now is
 // latency: 0.43 instructions a cycle and scheduler at 16 warps an SM.
 #pragma once
