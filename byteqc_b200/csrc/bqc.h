@@ -65,9 +65,51 @@ struct JKSub {
     int rows_are_b;    // tile rows run over the b list instead of the a list
     int row0;          // first tile row of the block among the launch's rows
     // parts a tile runs as (at least 1 each): ranges of its quartets (a power
-    // of two up to 8) and of the primitive ket pairs
+    // of two up to 8) and of the primitive quartets
     int rparts, kparts;
+    int kfirst;        // the range of the primitive quartets of a launch of one block
 };
+
+// A launch of one block runs whole tiles, or as many ranges of the primitive
+// quartets, one after another, as keep their length within 32 bits (four shells
+// of 216 primitives and more).
+inline void whole_prims(JKSub &s) {
+    s.rparts = 1;
+    s.kparts = (int)(((long long)s.nprim_a * s.nprim_b >> 31) + 1);
+}
+
+// Parts of the tiles of a class pair with many primitive quartets: a part
+// holds about PART_PRIMS primitive quartets per lane, first by fewer bra pairs
+// and then by a range of the primitives (the integrals are linear in it).  A
+// whole tile of two 6-primitive s pairs is 8 x 1296 primitive quartets in a
+// row, which no other work of a build hides: C60H122 / 6-31G**, (ss|ss) of both
+// precision bands, 32.9 -> 24.1 ms.  The schedule counts the parts of a tile row
+// in 32 bits, so the rows of a long pair list get fewer and longer parts.
+constexpr int PART_PRIMS = 64;
+
+inline void split_prims(JKSub &s) {
+    const long long n = (long long)s.nprim_a * s.nprim_b;
+    const long long cols = ((s.na > s.nb ? s.na : s.nb) + 15LL) / 16;
+    whole_prims(s);
+    while (s.rparts < 8 && 8 / s.rparts * n > PART_PRIMS && 2 * s.rparts * s.kparts * cols <= 0x7fffffffLL)
+        s.rparts *= 2;
+    const long long parts = n / PART_PRIMS + (n % PART_PRIMS != 0), most = 0x7fffffffLL / (cols * s.rparts);
+    if (parts > s.kparts) s.kparts = (int)(parts < most ? parts : most);
+}
+
+// Primitive quartets of range kpart of the kparts, bra pairs innermost: num from
+// the ket pair k and bra pair i on.  The product n * kpart passes 32 bits from
+// shells of 25 primitives on; undivided tiles take no division.
+struct PrimRange {
+    int k, i, num;
+};
+
+__host__ __device__ inline PrimRange prim_range(const JKSub &s, int kpart) {
+    if (s.kparts == 1) return {0, 0, s.nprim_a * s.nprim_b};
+    const long long n = (long long)s.nprim_a * s.nprim_b;
+    const long long begin = n * kpart / s.kparts, k = begin / s.nprim_a;
+    return {(int)k, (int)(begin - k * s.nprim_a), (int)(n * (kpart + 1) / s.kparts - begin)};
+}
 
 // the same block with bra and ket exchanged (a diagonal block has identical
 // lists on both sides; the a >= b rule stays)

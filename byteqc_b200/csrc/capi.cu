@@ -187,7 +187,7 @@ int GINTbuild_jk(BasisProdCache *bpcache, double *vj, double *vk, double *dm, in
         t.sub.pb0 = bpcache->primitive_pairs_locs[cp_kl_id] + kl0 * ckl->nprim_12;
         t.sub.nprim_a = cij->nprim_12;
         t.sub.nprim_b = ckl->nprim_12;
-        t.sub.rparts = t.sub.kparts = 1;
+        whole_prims(t.sub);
         t.sub.diag = cp_ij_id == cp_kl_id;
         int err = bqc_launch_jk(cij->l_bra, cij->l_ket, ckl->l_bra, ckl->l_ket, args, t, 0, stream);
         if (err) return err;
@@ -229,7 +229,7 @@ int GINTfill_int2e(BasisProdCache *bpcache, double *eri, int nao, int *strides, 
         t.sub.pb0 = bpcache->primitive_pairs_locs[cp_kl_id] + kl0 * ckl->nprim_12;
         t.sub.nprim_a = cij->nprim_12;
         t.sub.nprim_b = ckl->nprim_12;
-        t.sub.rparts = t.sub.kparts = 1;
+        whole_prims(t.sub);
         int err = bqc_launch_jk(cij->l_bra, cij->l_ket, ckl->l_bra, ckl->l_ket, args, t, 0, stream);
         if (err) return err;
     }
@@ -328,7 +328,7 @@ static int build_jk_band(const BasisProdCache *bp, JKArgs args, const double *pa
             s.pb0 = bp->primitive_pairs_locs[ckl];
             s.nprim_a = tij->nprim_12;
             s.nprim_b = tkl->nprim_12;
-            s.rparts = s.kparts = 1;
+            whole_prims(s);
             s.diag = cij == ckl;
             if (pair_q_host != nullptr) {
                 size_t off = prefix.size(), coff = col0.size();

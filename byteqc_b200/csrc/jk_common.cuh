@@ -39,9 +39,9 @@ __device__ __forceinline__ double dmax6(const double *__restrict__ dmc, int nbas
 // keeps the last one that qualifies, so a row index of up to 2^20 takes four
 // rounds of loads instead of twenty dependent ones.  All 32 lanes of every
 // warp must call it.
-// Every tile of a block runs as rparts * kparts parts: kpart of kparts ranges
-// of the primitive quartets, and one of rparts parts of its quartets; the
-// caller's (part, nparts) of the whole tile is refined by the latter.
+// Every tile of a launch over several blocks runs as rparts * kparts parts: kpart
+// of kparts ranges of the primitive quartets, and one of rparts parts of its
+// quartets; the caller's (part, nparts) of the whole tile is refined by the latter.
 __device__ __forceinline__ void tile_of_block(const JKTask &T, long long x, JKSub &s, int &r, int &c,
                                               int &part, int &nparts, int &kpart) {
     if (T.tile_prefix != nullptr) {
@@ -59,23 +59,25 @@ __device__ __forceinline__ void tile_of_block(const JKTask &T, long long x, JKSu
         const int y = (int)(x - __ldg(T.tile_prefix + r));   // a row's parts fit 32 bits
         const int col0 = T.tile_col0 != nullptr ? __ldg(T.tile_col0 + r) : 0;
         s = T.sub;
+        c = col0 + y;
+        kpart = s.kfirst;
         if (T.subs != nullptr) {
             s = T.subs[__ldg(T.row_sub + r)];
             r -= s.row0;
             if (T.swapped) s = jk_swap_sub(s);
+            const int parts = s.rparts * s.kparts;
+            c = col0 + y / parts;
+            const int p = y % parts;
+            kpart = p % s.kparts;
+            part = part * s.rparts + p / s.kparts;
+            nparts *= s.rparts;
         }
-        const int parts = s.rparts * s.kparts;
-        c = col0 + y / parts;
-        const int p = y % parts;
-        kpart = p % s.kparts;
-        part = part * s.rparts + p / s.kparts;
-        nparts *= s.rparts;
     } else {
         s = T.sub;
         const int ncols = ((s.rows_are_b ? s.na : s.nb) + TILE - 1) / TILE;
         r = (int)(x / ncols);
         c = (int)(x % ncols);
-        kpart = 0;
+        kpart = s.kfirst;
     }
 }
 

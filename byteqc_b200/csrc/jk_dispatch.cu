@@ -54,13 +54,16 @@ int bqc_launch_jk(int li, int lj, int lk, int ll, const JKArgs &args, const JKTa
     }
     int key = ((li * 4 + lj) * 4 + lk) * 4 + ll;
     int err = 0;
-    switch (key) {
+    const int ranges = t.subs == nullptr ? t.sub.kparts : 1;
+    for (t.sub.kfirst = 0; t.sub.kfirst < ranges && !err; t.sub.kfirst++) {
+        switch (key) {
 #define BQC_CASE(a, b, c, d) \
     case ((a * 4 + b) * 4 + c) * 4 + d: err = bqc_class_##a##b##c##d(a_, t, fp32, stream); break;
 #include "jk_classes.inc"
 #undef BQC_CASE
-    default:
-        return 2;
+        default:
+            return 2;
+        }
     }
     if (err) return err;
     cudaError_t ce = cudaGetLastError();

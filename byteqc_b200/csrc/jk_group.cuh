@@ -124,8 +124,7 @@ jk_group(JKArgs A, JKTask T) {
     int a_begin, b_begin, count, kpart;
     if (!tile_screen(A, T, x, s, s_list, &s_count, a_begin, b_begin, count, kpart, part, nparts)) return;
     // primitive quartets of this part
-    const int nprim = s.nprim_a * s.nprim_b;
-    const int p_begin = nprim * kpart / s.kparts, p_end = nprim * (kpart + 1) / s.kparts;
+    const PrimRange pr = prim_range(s, kpart);
 
     const int nrounds = (count + NG - 1) / NG;
     for (int round = 0; round < nrounds; round++) {
@@ -165,13 +164,14 @@ jk_group(JKArgs A, JKTask T) {
         };
         if (active && A.eri == nullptr) stage(A.dm);
 
-        for (int pr = p_begin; pr < p_end; pr++) {
+        int kp = pr.k, ip = pr.i;
+        for (int left = pr.num; left > 0; left--) {
             PrimQuartet P;
             if (active) {
-                const int kp = pr / s.nprim_a, ip = pr - kp * s.nprim_a;
                 PrimPair pi, pk;
                 load_prim(A, pa + ip, pi);
                 load_prim(A, pb + kp, pk);
+                if (++ip == s.nprim_a) { ip = 0; kp++; }
                 prim_quartet(pi, pk, bra.A, ket.A, fac, P);
                 for (int f = lane; f < 2 * NR; f += TPQ) rw[f] = rys_one<NR>(A.rys, P.x, f);
             }

@@ -140,9 +140,8 @@ jk_warp(JKArgs A, JKTask T) {
         // row steps of this part
         const int steps = max(ROW_STEPS / nparts, 1);
         const int it_end = min((part + 1) * steps, ROW_STEPS);
-        // primitive quartets [p_begin, p_end) of this part, bra pairs innermost
-        const int nprim = s.nprim_a * s.nprim_b;
-        const int p_begin = nprim * kpart / s.kparts, p_end = nprim * (kpart + 1) / s.kparts;
+        // primitive quartets of this part, bra pairs innermost
+        const PrimRange pr = prim_range(s, kpart);
         bool pending = false;                // the carried sums hold contributions
         auto bra_pair = [&](int it) { return min(a_begin + 2 * it + half, a_end - 1); };
         int a = bra_pair(part * steps);
@@ -178,10 +177,10 @@ jk_warp(JKArgs A, JKTask T) {
                 const F AB[3] = {F(bra.AB[0]), F(bra.AB[1]), F(bra.AB[2])};
                 const double fac = !active ? 0. : (a == b && A.eri == nullptr) ? 0.5 * TWO_PI_2P5 : TWO_PI_2P5;
                 const int pa = s.pa0 + (a - s.a0) * s.nprim_a;
-                int kp = p_begin / s.nprim_a, ip = p_begin - kp * s.nprim_a;
+                int kp = pr.k, ip = pr.i;
                 PrimPair pk;
                 load_prim(A, pb + kp, pk);
-                for (int left = p_end - p_begin; left > 0; left--) {
+                for (int left = pr.num; left > 0; left--) {
                     PrimPair pi;
                     load_prim(A, pa + ip, pi);
                     PrimQuartet P;

@@ -290,21 +290,6 @@ double prim_cost(int li, int lj, int lk, int ll) {
     return n * (15. * (li + lj + 1) * (lk + ll + 1) + 3. * nf) + 30.;
 }
 
-// Parts of the tiles of a class pair with many primitive quartets: a part
-// holds about PART_PRIMS primitive quartets per lane, first by fewer bra pairs
-// and then by a range of the primitives (the integrals are linear in it).  A
-// whole tile of two 6-primitive s pairs is 8 x 1296 primitive quartets in a
-// row, which no other work of a build hides: C60H122 / 6-31G**, (ss|ss) of both
-// precision bands, 32.9 -> 24.1 ms.
-constexpr int PART_PRIMS = 64;
-
-void split_prims(JKSub &s) {
-    const long long n = (long long)s.nprim_a * s.nprim_b;
-    s.rparts = 1;
-    while (s.rparts < 8 && 8 / s.rparts * n > PART_PRIMS) s.rparts *= 2;
-    s.kparts = n > PART_PRIMS ? (int)((n + PART_PRIMS - 1) / PART_PRIMS) : 1;
-}
-
 }  // namespace
 
 extern "C" {

@@ -460,6 +460,57 @@ def test_primitive_parts_match_whole_tiles(cuda, nc, n_dm, fp32_below):
         assert float((a - b).abs().max()) < tol
 
 
+def _contracted(shells, n):
+    """H2 with contracted shells [(l, number of primitives)] on each atom,
+    the second atom's exponents shifted."""
+    rng = np.random.default_rng(n)
+    basis = {}
+    for sym, shift in (('H', 1.), ('He', 1.3)):
+        basis[sym] = [[l] + [[shift * .08 * 400. ** (i / max(k - 1, 1)), float(rng.uniform(.2, 1.))]
+                             for i in range(k)] for l, k in shells]
+    return Mole([('H', (0., 0., 0.)), ('He', (.3, -.2, .7))], basis)
+
+
+@pytest.mark.parametrize('shells', [[(0, 25), (1, 1)], [(0, 3), (1, 3), (2, 3), (3, 3)], [(1, 2), (2, 7)]])
+def test_deep_contractions(cuda, shells):
+    """Ranges of the primitive quartets: 25^4 = 390,625 primitive quartets, the
+    first number whose products with the range index pass 32 bits, and the
+    contracted d and f classes of the group kernel.  J/K against the oracle and
+    the plan against the host-scheduled whole tiles, the latter as in
+    test_primitive_parts_match_whole_tiles."""
+    import ctypes
+    import torch
+    from byteqc_b200 import lib as L
+    from byteqc_b200.scf import hf
+    from byteqc_b200.scf.hf import _ptr, _stream
+    lib = L.load_library()
+    mol = _contracted(shells, 11)
+    opt = hf._VHFOpt(mol).build()
+    dm = _rand_dm(mol.nao, 9) * .1
+    vj, vk = hf.get_jk(mol, dm, vhfopt=opt)
+    rj, rk = oracle.get_jk(mol, dm)
+    scale = max(1., abs(rj).max() / 100)
+    print('deep %s: max|J| %.3g max|dJ| %.3e max|dK| %.3e' % (shells, abs(rj).max(), abs(vj - rj).max(), abs(vk - rk).max()))
+    assert abs(vj - rj).max() < TOL_JK * scale and abs(vk - rk).max() < TOL_JK * scale
+    C = opt.coeff_dev
+    dmc = (C @ torch.as_tensor(dm, device=cuda) @ C.T)[None].contiguous()
+    cond = torch.empty((opt.mol.nbas, opt.mol.nbas), dtype=torch.float64, device=cuda)
+    assert lib.BQCdm_cond(_ptr(dmc), 1, dmc.shape[-1], _ptr(opt._mem['ao_loc']), opt.mol.nbas, _ptr(cond),
+                          _stream()) == 0
+    wj, wk = torch.zeros_like(dmc), torch.zeros_like(dmc)
+    assert lib.BQCbuild_jk(ctypes.cast(opt.bpcache, ctypes.c_void_p), _ptr(opt.pair_q),
+                           opt.pair_q_host.ctypes.data_as(ctypes.c_void_p), _ptr(cond), float(cond.max()),
+                           _ptr(wj), _ptr(wk), _ptr(dmc), dmc.shape[-1], 1, opt.direct_scf_tol, 0., None,
+                           _stream()) == 0
+    pj, pk = torch.zeros_like(dmc), torch.zeros_like(dmc)
+    assert lib.BQCbuild_jk_plan(opt._plan, _ptr(opt.pair_q), _ptr(cond), _ptr(pj), _ptr(pk), _ptr(dmc),
+                                dmc.shape[-1], 1, opt.direct_scf_tol, 0., _stream()) == 0
+    torch.cuda.synchronize()
+    for a, b in ((wj, pj), (wk, pk)):
+        assert float(a.abs().max()) > 0
+        assert float((a - b).abs().max()) < 1e-12 * max(1., float(a.abs().max()))
+
+
 @pytest.mark.parametrize('kind,bra,ket', [('cc-pvdz', (2, 0), (1, 1)), ('cc-pvdz', (1, 1), (2, 2)),
                                           ('cc-pvdz', (1, 0), (2, 2)), ('cc-pvtz', (3, 0), (1, 1)),
                                           ('cc-pvtz', (1, 1), (3, 3)), ('cc-pvtz', (2, 0), (3, 3))])
