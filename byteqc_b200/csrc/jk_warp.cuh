@@ -255,6 +255,12 @@ jk_warp(JKArgs A, JKTask T) {
                 const double *__restrict__ D = A.dm + id * nn;
                 double *VJ = A.vj + id * nn, *VK = A.vk + id * nn;
                 if (any) {
+                    // J_ij and K_jk: summed over the lanes of a half warp
+                    double v[NIJ + NFJ * NFK];
+#pragma unroll
+                    for (int n = 0; n < NIJ + NFJ * NFK; n++) v[n] = 0.;
+                    // a lane that is screened out touches no density: it may hold anything
+                    if (active) {
                     // rows of the density: an element is one address step from its row
                     const double *Di[NFI], *Dj[NFJ], *Dk[NFK];
 #pragma unroll
@@ -263,10 +269,6 @@ jk_warp(JKArgs A, JKTask T) {
                     for (int n = 0; n < NFJ; n++) Dj[n] = D + (long long)(j0 + n) * nao;
 #pragma unroll
                     for (int n = 0; n < NFK; n++) Dk[n] = D + (long long)(k0 + n) * nao;
-                    // J_ij and K_jk: summed over the lanes of a half warp
-                    double v[NIJ + NFJ * NFK];
-#pragma unroll
-                    for (int n = 0; n < NIJ + NFJ * NFK; n++) v[n] = 0.;
                     if (A.vj != nullptr) {
 #pragma unroll
                         for (int kl = 0; kl < NKL; kl++) {
@@ -313,11 +315,9 @@ jk_warp(JKArgs A, JKTask T) {
 #pragma unroll
                                     for (int fl = 0; fl < NFL; fl++) pjl[fj * NFL + fl] += ACC(fi, fj, fk, fl) * d;
                             }
-                        if (active) {
 #pragma unroll
-                            for (int n = 0; n < NFJ * NFL; n++)
-                                atomicAdd(VK + (long long)(j0 + n / NFL) * kr + (long long)(l0 + n % NFL) * kc, pjl[n]);
-                        }
+                        for (int n = 0; n < NFJ * NFL; n++)
+                            atomicAdd(VK + (long long)(j0 + n / NFL) * kr + (long long)(l0 + n % NFL) * kc, pjl[n]);
                         // K_ik
                         double d_jl[NFJ * NFL];
 #pragma unroll
@@ -348,10 +348,11 @@ jk_warp(JKArgs A, JKTask T) {
                             // no shell k shared by the lanes: K_jk one by one
 #pragma unroll
                             for (int n = 0; n < NFJ * NFK; n++) {
-                                if (active) atomicAdd(VK + (long long)(j0 + n / NFK) * kr + (long long)(k0 + n % NFK) * kc, v[NIJ + n]);
+                                atomicAdd(VK + (long long)(j0 + n / NFK) * kr + (long long)(k0 + n % NFK) * kc, v[NIJ + n]);
                                 v[NIJ + n] = 0.;
                             }
                         }
+                    }
                     }
                     half_warp_sum(v, lane, [&](int n, double y) {
                         double *dst = n < NIJ ? VJ + (size_t)(i0 + n / NFJ) * nao + j0 + n % NFJ

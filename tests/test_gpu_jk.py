@@ -551,3 +551,54 @@ def test_stored_half_of_k(cuda, kind, bra, ket):
     cols = np.isin(l_of, ket)
     assert n > 0 and abs(K[np.ix_(rows, cols)]).max() > 0
     assert abs(K[~rows]).max() == 0 and abs(K[:, ~cols]).max() == 0
+
+
+@pytest.mark.parametrize('n_dm,fp32_below', [(1, 0.), (2, 0.), (1, 1e-6)])
+def test_screened_quartets_touch_no_density(cuda, n_dm, fp32_below):
+    """A quartet that is screened out contributes nothing, whatever the density
+    holds: with q = 0 for every pair of two shells (an s and a p shell, so that
+    every other quartet survives) NaN in their rows and columns leaves the
+    result as zeros there do.  Bound as in test_repeated_builds_agree."""
+    import ctypes
+    import torch
+    from byteqc_b200 import lib as L
+    from byteqc_b200.scf import hf
+    from byteqc_b200.scf.hf import _ptr, _stream
+    lib = L.load_library()
+    mol = _mol('cc-pvdz', nw=2, seed=31)
+    opt = hf._VHFOpt(mol).build()
+    C = opt.coeff_dev
+    dm = np.stack([_rand_dm(mol.nao, s) for s in range(n_dm)]) * .1
+    dmc = (C @ torch.as_tensor(dm, device=cuda) @ C.T).contiguous()
+    nao, loc = dmc.shape[-1], opt.mol.ao_loc_nr(cart=True)
+    l_of = opt.mol._bas[:, 1]
+    shells = [int(np.flatnonzero(l_of == 0)[2]), int(np.flatnonzero(l_of == 1)[1])]
+    rows = np.concatenate([np.arange(loc[s], loc[s + 1]) for s in shells])
+    q = opt.pair_q.clone()
+    q[torch.as_tensor(np.isin(opt.bas_pair2shls, shells).any(0), device=cuda)] = 0.
+    dmc[:, rows] = 0.
+    dmc[:, :, rows] = 0.
+    cond = torch.empty((opt.mol.nbas, opt.mol.nbas), dtype=torch.float64, device=cuda)
+    assert lib.BQCdm_cond(_ptr(dmc), n_dm, nao, _ptr(opt._mem['ao_loc']), opt.mol.nbas, _ptr(cond),
+                          _stream()) == 0
+    bad = dmc.clone()
+    bad[:, rows] = float('nan')
+    bad[:, :, rows] = float('nan')
+    for plan in (False, True):
+        out = []
+        for d in (dmc, bad):
+            vj, vk = torch.zeros_like(d), torch.zeros_like(d)
+            if plan:
+                err = lib.BQCbuild_jk_plan(opt._plan, _ptr(q), _ptr(cond), _ptr(vj), _ptr(vk), _ptr(d), nao,
+                                           n_dm, opt.direct_scf_tol, fp32_below, _stream())
+            else:
+                err = lib.BQCbuild_jk(ctypes.cast(opt.bpcache, ctypes.c_void_p), _ptr(q),
+                                      opt.pair_q_host.ctypes.data_as(ctypes.c_void_p), _ptr(cond),
+                                      float(cond.max()), _ptr(vj), _ptr(vk), _ptr(d), nao, n_dm,
+                                      opt.direct_scf_tol, fp32_below, None, _stream())
+            assert err == 0
+            out.append((vj, vk))
+        torch.cuda.synchronize()
+        for a, b in zip(*out):
+            assert float(a.abs().max()) > 0 and bool(torch.isfinite(b).all())
+            assert float((a - b).abs().max()) < 1e-13 * float(a.abs().max())
