@@ -14,7 +14,7 @@ struct JKArgs {
     const int *pair_bra;      // shell i of each pair        (bas_pair2bra)
     const int *pair_ket;      // shell j of each pair        (bas_pair2ket)
     const double *a12, *e12, *x12, *y12, *z12;  // primitive-pair data
-    // the same data as records (a plan keeps them; NULL otherwise): per pair
+    // the same data as records (made by the builds of a plan; NULL otherwise): per pair
     // PAIR_REC 16-byte words {shell i, shell j, ao_loc i, ao_loc j | A, A - B},
     // per primitive pair PRIM_REC words {a12, 1 / a12 | e12, x12 | y12, z12}
     const int4 *pair_rec;

@@ -8,7 +8,8 @@
 // schedule.  A build then runs entirely on the stream without a host
 // round trip or an allocation:
 //
-//   dm_max   = max over the density-block table (one reduction kernel);
+//   inputs   : dm_max = max over the density-block table, and the pair and
+//              primitive-pair records from the cache's arrays (one kernel);
 //   counts   : per tile row r of every task, the number of leading column
 //              tiles c with q_row[r] q_col[c] dm_max >= tol (the tiles are
 //              sorted by their first q, so a binary search), at most r + 1 on
@@ -147,13 +148,43 @@ __device__ __forceinline__ int first_mol(const int *__restrict__ mol, int lo, in
     return lo;
 }
 
-// max over the non-negative entries of x (as ordered 64-bit patterns)
-__global__ void max_kernel(const double *__restrict__ x, size_t n, unsigned long long *out) {
-    double m = 0.;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        m = fmax(m, __ldg(x + i));
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
+// What a build derives from its inputs first.  Blocks [0, max_blocks): the
+// maximum of the non-negative entries of x (as ordered 64-bit patterns).  The
+// others: the records of JKArgs::pair_rec and prim_rec from the cache's arrays as
+// they are at this point of the caller's stream.  Made by every build and not
+// once per plan: 112 bytes per pair and primitive pair are microseconds beside
+// its quartets, and the arrays may change between builds.
+__global__ void inputs_kernel(const double *__restrict__ x, size_t n, unsigned long long *out, int max_blocks,
+                              BasisProdCache bp, int npair, int nprim, int4 *__restrict__ pair_rec,
+                              double2 *__restrict__ prim_rec) {
+    if ((int)blockIdx.x < max_blocks) {
+        double m = 0.;
+        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)max_blocks * blockDim.x)
+            m = fmax(m, __ldg(x + i));
+        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
+        return;
+    }
+    const long long first = (blockIdx.x - max_blocks) * (long long)blockDim.x + threadIdx.x;
+    const long long step = (gridDim.x - max_blocks) * (long long)blockDim.x;
+    const double *cx = bp.bas_coords, *cy = cx + bp.nbas, *cz = cy + bp.nbas;
+    for (long long t = first; t < (long long)npair + nprim; t += step) {
+        if (t < npair) {
+            const int i = bp.bas_pair2bra[t], j = bp.bas_pair2ket[t];
+            int4 *r = pair_rec + t * PAIR_REC;
+            double2 *c = reinterpret_cast<double2 *>(r + 1);
+            r[0] = make_int4(i, j, bp.ao_loc[i], bp.ao_loc[j]);
+            c[0] = make_double2(cx[i], cy[i]);
+            c[1] = make_double2(cz[i], cx[i] - cx[j]);
+            c[2] = make_double2(cy[i] - cy[j], cz[i] - cz[j]);
+        } else {
+            const long long u = t - npair;
+            double2 *r = prim_rec + u * PRIM_REC;
+            r[0] = make_double2(bp.a12[u], 1.0 / bp.a12[u]);
+            r[1] = make_double2(bp.e12[u], bp.x12[u]);
+            r[2] = make_double2(bp.y12[u], bp.z12[u]);
+        }
+    }
 }
 
 // per global row: the column counts of the two precision bands (band 1 only
@@ -238,7 +269,7 @@ struct BQCPlan {
     int device;
     int nsm;
     std::vector<ShapeHost> shapes;   // costly first
-    int nshapes, nrows_all, npfx;
+    int nshapes, nrows_all, npfx, npair, nprim;
     SideStreams *streams;
     // device
     SchedTask *d_tasks;
@@ -257,29 +288,6 @@ struct BQCPlan {
 };
 
 namespace {
-
-// the records of JKArgs::pair_rec and prim_rec
-__global__ void pair_rec_kernel(BasisProdCache bp, int n, int4 *__restrict__ rec) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const int i = bp.bas_pair2bra[t], j = bp.bas_pair2ket[t];
-    const double *x = bp.bas_coords, *y = x + bp.nbas, *z = y + bp.nbas;
-    int4 *r = rec + (size_t)t * PAIR_REC;
-    double2 *c = reinterpret_cast<double2 *>(r + 1);
-    r[0] = make_int4(i, j, bp.ao_loc[i], bp.ao_loc[j]);
-    c[0] = make_double2(x[i], y[i]);
-    c[1] = make_double2(z[i], x[i] - x[j]);
-    c[2] = make_double2(y[i] - y[j], z[i] - z[j]);
-}
-
-__global__ void prim_rec_kernel(BasisProdCache bp, int n, double2 *__restrict__ rec) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    double2 *r = rec + (size_t)t * PRIM_REC;
-    r[0] = make_double2(bp.a12[t], 1.0 / bp.a12[t]);
-    r[1] = make_double2(bp.e12[t], bp.x12[t]);
-    r[2] = make_double2(bp.y12[t], bp.z12[t]);
-}
 
 // cost of one quartet of a class shape per primitive quartet (flops of the
 // Rys quadrature), to launch the costly shapes first
@@ -400,7 +408,8 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
     p->npfx = p->nrows_all + p->nshapes;
     const size_t nt = std::max<size_t>(st.size(), 1), nr = std::max(p->nrows_all, 1),
                  np_ = std::max(p->npfx, 1), ns = std::max(p->nshapes, 1);
-    const int npair = bp->bas_pairs_locs[bp->ncptype], nprim = bp->primitive_pairs_locs[bp->ncptype];
+    p->npair = bp->bas_pairs_locs[bp->ncptype];
+    p->nprim = bp->primitive_pairs_locs[bp->ncptype];
     bool ok = cudaMalloc(&p->d_tasks, sizeof(SchedTask) * nt) == cudaSuccess &&
               cudaMalloc(&p->d_shapes, sizeof(SchedShape) * ns) == cudaSuccess &&
               cudaMalloc(&p->d_subs, sizeof(JKSub) * nt) == cudaSuccess &&
@@ -411,8 +420,8 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
               cudaMalloc(&p->d_prefix, sizeof(long long) * 2 * np_) == cudaSuccess &&
               cudaMalloc(&p->d_ntiles, sizeof(long long) * 2 * ns) == cudaSuccess &&
               cudaMalloc(&p->d_dm_max, sizeof(unsigned long long)) == cudaSuccess &&
-              cudaMalloc(&p->d_pair_rec, sizeof(int4) * PAIR_REC * std::max(npair, 1)) == cudaSuccess &&
-              cudaMalloc(&p->d_prim_rec, sizeof(double2) * PRIM_REC * std::max(nprim, 1)) == cudaSuccess &&
+              cudaMalloc(&p->d_pair_rec, sizeof(int4) * PAIR_REC * std::max(p->npair, 1)) == cudaSuccess &&
+              cudaMalloc(&p->d_prim_rec, sizeof(double2) * PRIM_REC * std::max(p->nprim, 1)) == cudaSuccess &&
               (p->streams = take_side(p->device)) != nullptr;
     if (ok && pair_mol_host) ok = cudaMalloc(&p->d_tile_mol, sizeof(int) * tile_mol.size()) == cudaSuccess;
     if (ok && p->nshapes > 0)
@@ -429,13 +438,6 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
     if (ok && pair_mol_host)
         ok = cudaMemcpy(p->d_tile_mol, tile_mol.data(), sizeof(int) * tile_mol.size(),
                         cudaMemcpyHostToDevice) == cudaSuccess;
-    if (ok && npair > 0 && nprim > 0) {
-        // done before the plan is handed out: builds may come on any stream
-        pair_rec_kernel<<<(npair + 255) / 256, 256>>>(*bp, npair, p->d_pair_rec);
-        prim_rec_kernel<<<(nprim + 255) / 256, 256>>>(*bp, nprim, p->d_prim_rec);
-        bqc_count_launch(2);
-        ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess;
-    }
     if (!ok) {
         BQCplan_destroy(p);
         return 1;
@@ -475,11 +477,14 @@ int BQCbuild_jk_plan(const BQCPlan *p, const double *pair_q, const double *dm_co
     if (p->nshapes == 0) return 0;
     const BasisProdCache *bp = p->bp;
     const bool two = fp32_below > tol;
-    // 1. dm_max on the device
+    // 1. dm_max and the records on the device
     if (cudaMemsetAsync(p->d_dm_max, 0, sizeof(unsigned long long), stream) != cudaSuccess) return 1;
     const size_t nn = (size_t)bp->nbas * bp->nbas;
     bqc_count_launch(3);
-    max_kernel<<<std::min<size_t>(1024, (nn + 255) / 256), 256, 0, stream>>>(dm_cond, nn, p->d_dm_max);
+    const int max_blocks = (int)std::min<size_t>(1024, (nn + 255) / 256);
+    const int rec_blocks = (int)std::min(8LL * p->nsm, ((long long)p->npair + p->nprim) / 256 + 1);
+    inputs_kernel<<<max_blocks + rec_blocks, 256, 0, stream>>>(dm_cond, nn, p->d_dm_max, max_blocks, *bp,
+                                                               p->npair, p->nprim, p->d_pair_rec, p->d_prim_rec);
     // 2. column counts per row (band 0: FP64, bound >= fp32_below when two
     //    bands, else >= tol; band 1: FP32, bound >= tol) and their scans
     int *cnt0 = p->d_cnt, *cnt1 = p->d_cnt + std::max(p->nrows_all, 1);

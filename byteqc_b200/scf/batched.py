@@ -445,8 +445,9 @@ def _graphed(fn, example):
     """fn(x) -> (J, K) captured once as a CUDA graph over a static input
     shaped like example; the returned function copies its argument in,
     replays the graph and returns copies of the outputs.  The library's
-    launches all go to torch's current stream, which is the capture stream
-    inside torch.cuda.graph."""
+    launches go to torch's current stream, which is the capture stream
+    inside torch.cuda.graph, or to side streams of the plan that fork from
+    and join it, so the capture covers them."""
     static_in = example.clone()
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())

@@ -189,9 +189,15 @@ int BQCbuild_jk_noalloc(const BasisProdCache *bpcache, const double *pair_q, dou
  * descending within each tile of 16 pairs and along the tiles' first
  * pairs; pair_mol_host: the molecule of every pair for batched molecules,
  * else NULL).  BQCbuild_jk_plan then computes dm_max, the surviving 16 x 16
- * tiles of every class pair and their offsets on the device and launches
- * fixed grids that stride over them: no host work, no allocation and the
+ * tiles of every class pair and their offsets on the device and launches, per
+ * class shape, fixed grids that stride over them: no allocation and the
  * same launches every build, so a build can be captured in a CUDA graph.
+ * The launches run on side streams of the plan, which wait for what the caller's
+ * stream holds and which the caller's stream then waits for; the plan's
+ * scratch serves one build at a time.
+ * Creation reads host data only: the numbers and classes of the pairs and
+ * pair_q_host / pair_mol_host, which must stay as they are while the plan lives.
+ * The cache's device arrays are read by every build on the caller's stream.
  * Its results equal BQCbuild_jk's with the same arguments.  Returns 0, 1 on
  * a CUDA error, 2 for l > 3, 3 for missing arguments. */
 typedef struct BQCPlan BQCPlan;

@@ -602,3 +602,32 @@ def test_screened_quartets_touch_no_density(cuda, n_dm, fp32_below):
         for a, b in zip(*out):
             assert float(a.abs().max()) > 0 and bool(torch.isfinite(b).all())
             assert float((a - b).abs().max()) < 1e-13 * float(a.abs().max())
+
+
+def test_plan_reads_the_cache_at_the_build(cuda):
+    """A build takes the cache's device arrays as they are on the caller's
+    stream, as BQCbuild_jk does, not as they were when the plan was made: twice
+    the pair factors e12, written behind some milliseconds of other work, give
+    four times the integrals.  Bound as in test_repeated_builds_agree."""
+    import torch
+    from byteqc_b200.scf import hf
+    mol = _mol('cc-pvdz', nw=2, seed=41)
+    opt = hf._VHFOpt(mol).build()
+    dm = torch.as_tensor(_rand_dm(mol.nao, 5) * 0.1, device=cuda)[None]
+    ref = opt.jk_ao(dm)
+    torch.cuda.synchronize()
+    big = torch.ones((4096, 4096), dtype=torch.float64, device=cuda)
+    e12 = opt._mem['aexyz'].view(5, -1)[1]
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        for _ in range(3):
+            big = big @ big * 1e-4
+        e12 *= 2.
+        got = opt.jk_ao(dm)
+        e12 *= .5
+        again = opt.jk_ao(dm)
+    s.synchronize()
+    for a, b, c in zip(ref, got, again):
+        assert float((4. * a - b).abs().max()) < 1e-13 * float(b.abs().max())
+        assert float((a - c).abs().max()) < 1e-13 * float(a.abs().max())
