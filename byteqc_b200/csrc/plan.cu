@@ -48,52 +48,81 @@ constexpr int TILE = 16;
 // Side streams of a plan: as many as a process has hardware queues by default.
 constexpr int SIDE_STREAMS = 8;
 
-struct SideStreams {
+// What a plan takes from the device beside its caller's streams: side streams with
+// their events, and one allocation for all its arrays.
+struct Resources {
     cudaStream_t side[SIDE_STREAMS];
     cudaEvent_t fork, join[SIDE_STREAMS];
+    char *slab;
+    size_t bytes;
 };
 
-// Creating the streams and events takes 0.6-1 ms, as long as the rest of a
-// small molecule's set-up: a destroyed plan's set is kept for the next plan on
-// its device, at most SETS_KEPT of them.  A set belongs to one plan at a time.
-constexpr size_t SETS_KEPT = 4;
+// Creating the streams and events takes 0.5 ms, an allocation of a few MB 1.4
+// ms, as long as the rest of a small molecule's set-up: what a destroyed plan
+// had is kept for the next plan on its device, at most SETS_KEPT sets of at most
+// SLAB_KEPT bytes.  A set belongs to one plan at a time.  _VHFOpt.build() of
+// geometries after one another, with an allocation for each array and none kept
+// and now: four waters / cc-pVDZ 4.1 -> 3.75 ms, a 20-carbon chain / 6-31G** 17.0 ->
+// 15.2 ms.
+constexpr size_t SETS_KEPT = 4, SLAB_KEPT = 64 << 20;
 std::mutex g_sets_lock;
-std::vector<std::pair<int, SideStreams *>> g_sets;   // (device, idle set)
+std::vector<std::pair<int, Resources *>> g_sets;   // (device, idle set)
 
-void free_side(SideStreams *s) {
+void free_set(Resources *s) {
     for (int n = 0; n < SIDE_STREAMS; n++) {
         if (s->side[n]) cudaStreamDestroy(s->side[n]);
         if (s->join[n]) cudaEventDestroy(s->join[n]);
     }
     if (s->fork) cudaEventDestroy(s->fork);
+    cudaFree(s->slab);
     delete s;
 }
 
-SideStreams *take_side(int device) {
+// an idle set of the device, the smallest that holds `bytes` if one does, or a new one
+Resources *take_set(int device, size_t bytes) {
+    Resources *s = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_sets_lock);
-        for (size_t n = 0; n < g_sets.size(); n++) {
-            if (g_sets[n].first == device) {
-                SideStreams *s = g_sets[n].second;
-                g_sets.erase(g_sets.begin() + n);
-                return s;
-            }
+        auto best = g_sets.end();
+        for (auto it = g_sets.begin(); it != g_sets.end(); ++it) {
+            if (it->first != device) continue;
+            const size_t have = it->second->bytes, most = best == g_sets.end() ? 0 : best->second->bytes;
+            if (best == g_sets.end() || (have >= bytes ? most < bytes || have < most : have > most)) best = it;
+        }
+        if (best != g_sets.end()) {
+            s = best->second;
+            g_sets.erase(best);
         }
     }
-    SideStreams *s = new SideStreams();   // value-initialised: every handle NULL
-    bool ok = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess;
-    for (int n = 0; ok && n < SIDE_STREAMS; n++)
-        ok = cudaStreamCreateWithFlags(&s->side[n], cudaStreamNonBlocking) == cudaSuccess &&
-             cudaEventCreateWithFlags(&s->join[n], cudaEventDisableTiming) == cudaSuccess;
+    bool ok = true;
+    if (s == nullptr) {
+        s = new Resources();   // value-initialised: every handle NULL
+        ok = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess;
+        for (int n = 0; ok && n < SIDE_STREAMS; n++)
+            ok = cudaStreamCreateWithFlags(&s->side[n], cudaStreamNonBlocking) == cudaSuccess &&
+                 cudaEventCreateWithFlags(&s->join[n], cudaEventDisableTiming) == cudaSuccess;
+    }
+    if (ok && s->bytes < bytes) {
+        cudaFree(s->slab);
+        s->slab = nullptr;
+        s->bytes = 0;
+        ok = cudaMalloc(&s->slab, bytes) == cudaSuccess;
+        if (ok) s->bytes = bytes;
+    }
     if (!ok) {
-        free_side(s);
+        free_set(s);
         return nullptr;
     }
     return s;
 }
 
-void give_side(int device, SideStreams *s) {
-    if (s == nullptr) return;
+// back from a plan, nothing of which may be in flight any more
+void give_set(int device, Resources *s) {
+    if (s->bytes > SLAB_KEPT) {
+        cudaFree(s->slab);
+        s->slab = nullptr;
+        s->bytes = 0;
+    }
     {
         std::lock_guard<std::mutex> lock(g_sets_lock);
         if (g_sets.size() < SETS_KEPT) {
@@ -101,7 +130,7 @@ void give_side(int device, SideStreams *s) {
             return;
         }
     }
-    free_side(s);
+    free_set(s);
 }
 
 // density-independent description of one class pair for the schedule kernels
@@ -270,8 +299,8 @@ struct BQCPlan {
     int nsm;
     std::vector<ShapeHost> shapes;   // costly first
     int nshapes, nrows_all, npfx, npair, nprim;
-    SideStreams *streams;
-    // device
+    Resources *res;
+    // device: parts of the set's allocation
     SchedTask *d_tasks;
     SchedShape *d_shapes;
     JKSub *d_subs;
@@ -410,38 +439,51 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
                  np_ = std::max(p->npfx, 1), ns = std::max(p->nshapes, 1);
     p->npair = bp->bas_pairs_locs[bp->ncptype];
     p->nprim = bp->primitive_pairs_locs[bp->ncptype];
-    bool ok = cudaMalloc(&p->d_tasks, sizeof(SchedTask) * nt) == cudaSuccess &&
-              cudaMalloc(&p->d_shapes, sizeof(SchedShape) * ns) == cudaSuccess &&
-              cudaMalloc(&p->d_subs, sizeof(JKSub) * nt) == cudaSuccess &&
-              cudaMalloc(&p->d_row_task, sizeof(int) * nr) == cudaSuccess &&
-              cudaMalloc(&p->d_tile_q, sizeof(double) * tile_q.size()) == cudaSuccess &&
-              cudaMalloc(&p->d_cnt, sizeof(int) * 2 * nr) == cudaSuccess &&
-              cudaMalloc(&p->d_col0, sizeof(int) * nr) == cudaSuccess &&
-              cudaMalloc(&p->d_prefix, sizeof(long long) * 2 * np_) == cudaSuccess &&
-              cudaMalloc(&p->d_ntiles, sizeof(long long) * 2 * ns) == cudaSuccess &&
-              cudaMalloc(&p->d_dm_max, sizeof(unsigned long long)) == cudaSuccess &&
-              cudaMalloc(&p->d_pair_rec, sizeof(int4) * PAIR_REC * std::max(p->npair, 1)) == cudaSuccess &&
-              cudaMalloc(&p->d_prim_rec, sizeof(double2) * PRIM_REC * std::max(p->nprim, 1)) == cudaSuccess &&
-              (p->streams = take_side(p->device)) != nullptr;
-    if (ok && pair_mol_host) ok = cudaMalloc(&p->d_tile_mol, sizeof(int) * tile_mol.size()) == cudaSuccess;
-    if (ok && p->nshapes > 0)
-        ok = cudaMemcpy(p->d_tasks, st.data(), sizeof(SchedTask) * st.size(), cudaMemcpyHostToDevice) == cudaSuccess &&
-             cudaMemcpy(p->d_shapes, ss.data(), sizeof(SchedShape) * ss.size(), cudaMemcpyHostToDevice) ==
-                 cudaSuccess &&
-             cudaMemcpy(p->d_subs, subs.data(), sizeof(JKSub) * subs.size(), cudaMemcpyHostToDevice) ==
-                 cudaSuccess &&
-             cudaMemcpy(p->d_row_task, row_task.data(), sizeof(int) * row_task.size(),
-                        cudaMemcpyHostToDevice) == cudaSuccess;
-    if (ok)
-        ok = cudaMemcpy(p->d_tile_q, tile_q.data(), sizeof(double) * tile_q.size(), cudaMemcpyHostToDevice) ==
-             cudaSuccess;
-    if (ok && pair_mol_host)
-        ok = cudaMemcpy(p->d_tile_mol, tile_mol.data(), sizeof(int) * tile_mol.size(),
-                        cudaMemcpyHostToDevice) == cudaSuccess;
-    if (!ok) {
+    // One allocation: what the schedule reads, uploaded in one copy, then the scratch
+    size_t bytes = 0;
+    auto part = [&bytes](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    };
+    const size_t tasks = part(sizeof(SchedTask) * nt), shapes = part(sizeof(SchedShape) * ns),
+                 subs_at = part(sizeof(JKSub) * nt), rows = part(sizeof(int) * nr),
+                 tq = part(sizeof(double) * tile_q.size()), tm = part(sizeof(int) * tile_mol.size()),
+                 upload = bytes;
+    const size_t cnt = part(sizeof(int) * 2 * nr), col0 = part(sizeof(int) * nr),
+                 prefix = part(sizeof(long long) * 2 * np_), ntiles = part(sizeof(long long) * 2 * ns),
+                 dm_max = part(sizeof(unsigned long long)),
+                 pair_rec = part(sizeof(int4) * PAIR_REC * std::max(p->npair, 1)),
+                 prim_rec = part(sizeof(double2) * PRIM_REC * std::max(p->nprim, 1));
+    std::vector<char> host(upload);
+    auto fill = [&host](size_t at, const auto &v) {
+        if (!v.empty()) memcpy(host.data() + at, v.data(), sizeof(v[0]) * v.size());
+    };
+    fill(tasks, st);
+    fill(shapes, ss);
+    fill(subs_at, subs);
+    fill(rows, row_task);
+    fill(tq, tile_q);
+    fill(tm, tile_mol);
+    p->res = take_set(p->device, bytes);
+    if (p->res == nullptr || cudaMemcpy(p->res->slab, host.data(), upload, cudaMemcpyHostToDevice) != cudaSuccess) {
         BQCplan_destroy(p);
         return 1;
     }
+    char *slab = p->res->slab;
+    p->d_tasks = (SchedTask *)(slab + tasks);
+    p->d_shapes = (SchedShape *)(slab + shapes);
+    p->d_subs = (JKSub *)(slab + subs_at);
+    p->d_row_task = (int *)(slab + rows);
+    p->d_tile_q = (double *)(slab + tq);
+    p->d_tile_mol = pair_mol_host ? (int *)(slab + tm) : nullptr;
+    p->d_cnt = (int *)(slab + cnt);
+    p->d_col0 = (int *)(slab + col0);
+    p->d_prefix = (long long *)(slab + prefix);
+    p->d_ntiles = (long long *)(slab + ntiles);
+    p->d_dm_max = (unsigned long long *)(slab + dm_max);
+    p->d_pair_rec = (int4 *)(slab + pair_rec);
+    p->d_prim_rec = (double2 *)(slab + prim_rec);
     // costly shapes first, so that the cheap ones fill the tail
     // (the rows and prefixes stay in the order of the device arrays)
     for (int n = 0; n < p->nshapes; n++) p->shapes[n].index = n;
@@ -453,20 +495,15 @@ int BQCplan_create(const BasisProdCache *bp, const double *pair_q_host, const in
 
 void BQCplan_destroy(BQCPlan *p) {
     if (p == nullptr) return;
-    cudaFree(p->d_tasks);   // waits for the plan's launches
-    cudaFree(p->d_shapes);
-    cudaFree(p->d_subs);
-    cudaFree(p->d_row_task);
-    cudaFree(p->d_tile_q);
-    cudaFree(p->d_tile_mol);
-    cudaFree(p->d_cnt);
-    cudaFree(p->d_col0);
-    cudaFree(p->d_prefix);
-    cudaFree(p->d_ntiles);
-    cudaFree(p->d_dm_max);
-    cudaFree(p->d_pair_rec);
-    cudaFree(p->d_prim_rec);
-    give_side(p->device, p->streams);
+    if (p->res != nullptr) {
+        // the plan's launches end before its set serves another plan
+        int dev = p->device;
+        cudaGetDevice(&dev);
+        if (dev != p->device) cudaSetDevice(p->device);
+        cudaDeviceSynchronize();
+        if (dev != p->device) cudaSetDevice(dev);
+        give_set(p->device, p->res);
+    }
     delete p;
 }
 
@@ -522,7 +559,7 @@ int BQCbuild_jk_plan(const BQCPlan *p, const double *pair_q, const double *dm_co
     args.rys = bqc_rys_table();
     args.rys_lm = bqc_rys_table_lm();
     // fork: the shapes are independent (the outputs are accumulated by atomics)
-    const SideStreams &ss = *p->streams;
+    const Resources &ss = *p->res;
     if (cudaEventRecord(ss.fork, stream) != cudaSuccess) return 1;
     for (int n = 0; n < SIDE_STREAMS; n++)
         if (cudaStreamWaitEvent(ss.side[n], ss.fork, 0) != cudaSuccess) return 1;

@@ -631,3 +631,40 @@ def test_plan_reads_the_cache_at_the_build(cuda):
     for a, b, c in zip(ref, got, again):
         assert float((4. * a - b).abs().max()) < 1e-13 * float(b.abs().max())
         assert float((a - c).abs().max()) < 1e-13 * float(a.abs().max())
+
+
+def test_plans_at_once_and_after_one_another(cuda):
+    """Two plans' builds in flight on two streams, one plan destroyed and its
+    streams and memory taken by a larger and by a smaller molecule's, more plans
+    alive than sets are kept: each gives its own result.  Bound as in
+    test_repeated_builds_agree."""
+    import torch
+    from byteqc_b200.scf import hf
+    mols = [_mol('cc-pvdz', nw=n, seed=50 + n) for n in (1, 3, 2)]
+    dms = [torch.as_tensor(_rand_dm(m.nao, n) * .1, device=cuda)[None] for n, m in enumerate(mols)]
+    refs = [hf._VHFOpt(m).build().jk_ao(d) for m, d in zip(mols, dms)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in mols]
+
+    def start(n, opt):
+        with torch.cuda.stream(streams[n]):
+            return opt.jk_ao(dms[n])
+
+    def check(n, out):
+        streams[n].synchronize()
+        for a, b in zip(refs[n], out):
+            assert float((a - b).abs().max()) < 1e-13 * float(a.abs().max())
+    for first, second, third in ((0, 1, 2), (1, 2, 0), (2, 0, 1)):
+        a, b = hf._VHFOpt(mols[first]).build(), hf._VHFOpt(mols[second]).build()
+        out_a, out_b = start(first, a), start(second, b)
+        a.clear()
+        c = hf._VHFOpt(mols[third]).build()
+        out_c, again_b = start(third, c), start(second, b)
+        check(first, out_a)
+        check(second, out_b)
+        check(second, again_b)
+        check(third, out_c)
+    many = [hf._VHFOpt(mols[n % 3]).build() for n in range(6)]
+    outs = [start(n % 3, opt) for n, opt in enumerate(many)]
+    for n, out in enumerate(outs):
+        check(n % 3, out)
