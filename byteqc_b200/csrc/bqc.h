@@ -150,6 +150,9 @@ struct JKTask {
     // grid holds at most a few CTAs per SM of the nsm SMs.
     const long long *ntiles_dev;
     int nsm;
+    // priority of the launch (0: that of its stream): side streams have the
+    // default one, their launches that of the caller's stream
+    int priority;
     // parts per tile of a launch without ntiles_dev (set by the
     // launcher; with ntiles_dev the kernel derives it from the device count)
     int split;

@@ -234,6 +234,22 @@ static int smem_attr(int bytes) {
     return 0;
 }
 
+// One launch at the task's priority; errors are left to cudaGetLastError().
+static inline void launch_at(void (*kernel)(JKArgs, JKTask), int grid, int block, size_t smem, cudaStream_t stream,
+                             const JKArgs &args, const JKTask &task) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributePriority;
+    attr.val.priority = task.priority;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = task.priority != 0;
+    cudaLaunchKernelEx(&cfg, kernel, args, task);
+}
+
 // SM count of the current device (cached per device; 0 on error)
 static inline int device_sms() {
     static std::atomic<int> sms[MAX_DEVICES];

@@ -449,7 +449,7 @@ static int launch_group_f(const JKArgs &args, const JKTask &task, cudaStream_t s
     t.split = group_split(t.ntiles, t.nsm);
     // with a device tile count the kernel cuts tiles into at most 8 parts
     const int grid = t.ntiles_dev == nullptr ? bqc_grid(t, t.ntiles, t.split, 0) : bqc_grid(t, t.ntiles, 8, 8);
-    jk_group<LI, LJ, LK, LL, TJ, NSPLIT, F><<<grid, C::NT, C::SMEM, stream>>>(args, t);
+    launch_at(jk_group<LI, LJ, LK, LL, TJ, NSPLIT, F>, grid, C::NT, C::SMEM, stream, args, t);
     return 0;
 }
 

@@ -427,7 +427,7 @@ static int launch_warp_range(const JKArgs &args, const JKTask &task, cudaStream_
                          : bqc_grid(task, task.ntiles, ROW_STEPS / WARPS, cap);
     constexpr int smem = WarpCfg<LI, LJ, LK, LL, KN>::SMEM;
     if (smem > 48 * 1024 && smem_attr<jk_warp<LI, LJ, LK, LL, F, K0, KN>>(smem)) return 1;
-    jk_warp<LI, LJ, LK, LL, F, K0, KN><<<grid, WARP_CTA, smem, stream>>>(args, task);
+    launch_at(jk_warp<LI, LJ, LK, LL, F, K0, KN>, grid, WARP_CTA, smem, stream, args, task);
     return 0;
 }
 

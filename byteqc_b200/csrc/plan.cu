@@ -558,6 +558,8 @@ int BQCbuild_jk_plan(const BQCPlan *p, const double *pair_q, const double *dm_co
     args.n_dm = n_dm;
     args.rys = bqc_rys_table();
     args.rys_lm = bqc_rys_table_lm();
+    int priority = 0;
+    if (cudaStreamGetPriority(stream, &priority) != cudaSuccess) return 1;
     // fork: the shapes are independent (the outputs are accumulated by atomics)
     const Resources &ss = *p->res;
     if (cudaEventRecord(ss.fork, stream) != cudaSuccess) return 1;
@@ -580,6 +582,7 @@ int BQCbuild_jk_plan(const BQCPlan *p, const double *pair_q, const double *dm_co
             t.row_sub = p->d_row_task + h.row0;
             t.ntiles_dev = p->d_ntiles + (size_t)band * p->nshapes + h.index;
             t.nsm = p->nsm;
+            t.priority = priority;
             err = bqc_launch_jk(h.li, h.lj, h.lk, h.ll, a, t, band == 1, ss.side[turn++ % SIDE_STREAMS]);
         }
     }

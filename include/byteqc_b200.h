@@ -193,8 +193,8 @@ int BQCbuild_jk_noalloc(const BasisProdCache *bpcache, const double *pair_q, dou
  * class shape, fixed grids that stride over them: no allocation and the
  * same launches every build, so a build can be captured in a CUDA graph.
  * The launches run on side streams of the plan, which wait for what the caller's
- * stream holds and which the caller's stream then waits for; the plan's
- * scratch serves one build at a time.
+ * stream holds and which the caller's stream then waits for, at the priority
+ * of the caller's stream; the plan's scratch serves one build at a time.
  * Creation reads host data only: the numbers and classes of the pairs and
  * pair_q_host / pair_mol_host, which must stay as they are while the plan lives.
  * The cache's device arrays are read by every build on the caller's stream.

@@ -668,3 +668,42 @@ def test_plans_at_once_and_after_one_another(cuda):
     outs = [start(n % 3, opt) for n, opt in enumerate(many)]
     for n, out in enumerate(outs):
         check(n % 3, out)
+
+
+def test_build_keeps_the_priority_of_the_callers_stream(cuda):
+    """The launches on the side streams run at the priority of the caller's
+    stream: read off the kernel nodes of a captured build."""
+    import torch
+    from cuda.bindings import runtime as rt
+    from byteqc_b200 import lib as L
+    from byteqc_b200.scf import hf
+    from byteqc_b200.scf.hf import _ptr
+    import ctypes
+    lib = L.load_library()
+    mol = _mol('cc-pvdz', nw=1, seed=2)
+    opt = hf._VHFOpt(mol).build()
+    C = opt.coeff_dev
+    dmc = (C @ torch.as_tensor(_rand_dm(mol.nao), device=cuda) @ C.T)[None].contiguous()
+    cond = torch.ones((opt.mol.nbas, opt.mol.nbas), dtype=torch.float64, device=cuda)
+    vj, vk = torch.zeros_like(dmc), torch.zeros_like(dmc)
+    def build(s):
+        assert lib.BQCbuild_jk_plan(opt._plan, _ptr(opt.pair_q), _ptr(cond), _ptr(vj), _ptr(vk), _ptr(dmc),
+                                    dmc.shape[-1], 1, opt.direct_scf_tol, 1e-6, ctypes.c_void_p(s.cuda_stream)) == 0
+    for priority in (0, -1):
+        s = torch.cuda.Stream(priority=priority)
+        s.wait_stream(torch.cuda.current_stream())
+        build(s)
+        s.synchronize()
+        mode = rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal
+        assert rt.cudaStreamBeginCapture(s.cuda_stream, mode)[0] == 0
+        build(s)
+        err, graph = rt.cudaStreamEndCapture(s.cuda_stream)
+        assert err == 0
+        _, _, n = rt.cudaGraphGetNodes(graph)
+        _, nodes, n = rt.cudaGraphGetNodes(graph, n)
+        kernels = [x for x in nodes[:n]
+                   if rt.cudaGraphNodeGetType(x)[1] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel]
+        got = [rt.cudaGraphKernelNodeGetAttribute(x, rt.cudaLaunchAttributeID.cudaLaunchAttributePriority)[1].priority
+               for x in kernels]
+        assert rt.cudaGraphDestroy(graph)[0] == 0
+        assert len(got) > 20 and set(got) == {priority}
