@@ -234,7 +234,8 @@ static int smem_attr(int bytes) {
     return 0;
 }
 
-// One launch at the task's priority; errors are left to cudaGetLastError().
+// One launch, at the task's priority if it has one; errors are left to
+// cudaGetLastError().
 static inline void launch_at(void (*kernel)(JKArgs, JKTask), int grid, int block, size_t smem, cudaStream_t stream,
                              const JKArgs &args, const JKTask &task) {
     cudaLaunchAttribute attr;
@@ -246,7 +247,7 @@ static inline void launch_at(void (*kernel)(JKArgs, JKTask), int grid, int block
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &attr;
-    cfg.numAttrs = task.priority != 0;
+    cfg.numAttrs = task.ntiles_dev != nullptr && task.priority != 0;
     cudaLaunchKernelEx(&cfg, kernel, args, task);
 }
 

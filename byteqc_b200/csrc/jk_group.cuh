@@ -446,7 +446,7 @@ static int launch_group_f(const JKArgs &args, const JKTask &task, cudaStream_t s
     if (t.ntiles == 0) return 0;
     if (smem_attr<jk_group<LI, LJ, LK, LL, TJ, NSPLIT, F>>((int)C::SMEM)) return 1;
     if (t.nsm <= 0 && (t.nsm = device_sms()) <= 0) return 1;
-    t.split = group_split(t.ntiles, t.nsm);
+    if (t.ntiles_dev == nullptr) t.split = group_split(t.ntiles, t.nsm);
     // with a device tile count the kernel cuts tiles into at most 8 parts
     const int grid = t.ntiles_dev == nullptr ? bqc_grid(t, t.ntiles, t.split, 0) : bqc_grid(t, t.ntiles, 8, 8);
     launch_at(jk_group<LI, LJ, LK, LL, TJ, NSPLIT, F>, grid, C::NT, C::SMEM, stream, args, t);

@@ -421,9 +421,8 @@ jk_warp(JKArgs A, JKTask T) {
 template <int LI, int LJ, int LK, int LL, typename F, int K0, int KN>
 static int launch_warp_range(const JKArgs &args, const JKTask &task, cudaStream_t stream) {
     constexpr int cap = 4 * WarpCfg<LI, LJ, LK, LL, KN>::MINB;   // persistent CTAs per SM
-    const long long n = (task.ntiles * task.split + WARPS - 1) / WARPS;
     const int grid = task.ntiles_dev == nullptr
-                         ? bqc_grid(task, n, 1, 0)
+                         ? bqc_grid(task, (task.ntiles * task.split + WARPS - 1) / WARPS, 1, 0)
                          : bqc_grid(task, task.ntiles, ROW_STEPS / WARPS, cap);
     constexpr int smem = WarpCfg<LI, LJ, LK, LL, KN>::SMEM;
     if (smem > 48 * 1024 && smem_attr<jk_warp<LI, LJ, LK, LL, F, K0, KN>>(smem)) return 1;
@@ -449,7 +448,7 @@ static int launch_warp(const JKArgs &args, const JKTask &task, int fp32, cudaStr
     t.ntiles = task_tiles(task);
     if (t.ntiles == 0) return 0;
     if (t.nsm <= 0 && (t.nsm = device_sms()) <= 0) return 1;
-    t.split = warp_split(t.ntiles, t.nsm);
+    if (t.ntiles_dev == nullptr) t.split = warp_split(t.ntiles, t.nsm);
     bqc_count_launch(cdiv(ncart(LK), CK) - 1);   // the dispatcher counted one
     if (fp32) return launch_warp_f<LI, LJ, LK, LL, float, 0, CK>(args, t, stream);
     return launch_warp_f<LI, LJ, LK, LL, double, 0, CK>(args, t, stream);
