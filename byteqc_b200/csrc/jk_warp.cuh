@@ -60,12 +60,16 @@ __device__ __forceinline__ void half_warp_sum(double (&v)[V], int lane, Emit emi
         if (n < cnt && v[n] != 0) emit(off + n, v[n]);
 }
 
+constexpr int LARGE_NF = 54;   // blocks of so many components fill the registers
+
 template <int LI, int LJ, int LK, int LL, int KN>
 struct WarpCfg {
     static constexpr int NFI = ncart(LI), NFJ = ncart(LJ), NFK = KN, NFL = ncart(LL);
     static constexpr int NF = NFI * NFJ * NFK * NFL;
     // sums carried over the bra pairs of a tile: J_kl, K_il, K_ik
     static constexpr int PERS = NFK * NFL + NFI * NFL + NFI * NFK;
+    // sums over a half warp: J_ij, K_jk
+    static constexpr int RED = NFI * NFJ + NFJ * NFK;
     // in registers beside the quartet block where both fit (64 doubles are half
     // of the largest register budget), else in shared memory, one column per
     // lane, which no other lane touches
@@ -454,12 +458,18 @@ static int launch_warp(const JKArgs &args, const JKTask &task, int fp32, cudaStr
     return launch_warp_f<LI, LJ, LK, LL, double, 0, CK>(args, t, stream);
 }
 
-// A class of at most SMALL_NF components.  The lanes hold the ket pairs and
-// carry J_kl, K_il and K_ik over the bra pairs: of the two orientations the
-// one that carries fewer sums.
+// A class of at most SMALL_NF components, in one of its two orientations.  The
+// lanes hold the ket pairs and carry J_kl, K_il and K_ik over the bra pairs:
+// the orientation that carries fewer sums.  From LARGE_NF components on it is the
+// one with fewer sums over the half warp, whose vector is live with the block:
+// one build of (H2O)_32 / cc-pVDZ, (dp|ps) with 9 of them 3.6 ms, with 27 3.9 ms,
+// (ds|pp) 2.2 and 2.4 ms.  Below, the carried sums cost more: (pp|ss) 5.1 ms
+// with 4 of them and 15 carried, 4.6 ms with 12 and 7, (pp|ps) 6.1 and 5.6 ms.
 template <int L1, int L2, int L3, int L4>
 static int launch_small(const JKArgs &args, const JKTask &task, int fp32, cudaStream_t stream) {
-    if constexpr (WarpCfg<L3, L4, L1, L2, ncart(L1)>::PERS < WarpCfg<L1, L2, L3, L4, ncart(L3)>::PERS) {
+    using C = WarpCfg<L1, L2, L3, L4, ncart(L3)>;
+    using S = WarpCfg<L3, L4, L1, L2, ncart(L1)>;
+    if constexpr (C::NF < LARGE_NF ? S::PERS < C::PERS : S::RED < C::RED) {
         JKTask sw = jk_swap_task(task);
         sw.k_transposed = !sw.k_transposed;
         return launch_warp<L3, L4, L1, L2, ncart(L1)>(jk_args_swap_eri(args), sw, fp32, stream);

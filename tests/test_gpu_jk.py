@@ -511,7 +511,8 @@ def test_deep_contractions(cuda, shells):
         assert float((a - b).abs().max()) < 1e-12 * max(1., float(a.abs().max()))
 
 
-@pytest.mark.parametrize('kind,bra,ket', [('cc-pvdz', (2, 0), (1, 1)), ('cc-pvdz', (1, 1), (2, 2)),
+@pytest.mark.parametrize('kind,bra,ket', [('cc-pvdz', (2, 0), (1, 1)), ('cc-pvdz', (2, 1), (1, 0)),
+                                          ('cc-pvdz', (1, 1), (2, 2)),
                                           ('cc-pvdz', (1, 0), (2, 2)), ('cc-pvtz', (3, 0), (1, 1)),
                                           ('cc-pvtz', (1, 1), (3, 3)), ('cc-pvtz', (2, 0), (3, 3))])
 def test_stored_half_of_k(cuda, kind, bra, ket):
