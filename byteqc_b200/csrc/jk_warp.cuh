@@ -8,10 +8,11 @@
 // 16 lanes, and only D_jl, its bound and the atomic on K_jl are per quartet;
 // the 128-thread half tiles that this replaces read all of it per quartet
 // (77 % of the L1 wavefront peak for (ps|ss)) and met at block barriers.
-// Measured on B200, one build of (H2O)_32 / cc-pVDZ: (ps|ss) 18.7 -> 14.3 ms,
-// (ss|ss) 10.3 -> 6.7 ms, (ps|ps) 11.6 -> 8.7 ms, (ds|ds) 1.10 -> 0.74 ms, but
-// (dp|ps) 4.1 -> 4.2 ms and (ds|pp) 2.3 -> 2.6 ms.  What bounds it now is
-// latency: 0.43 instructions a cycle and scheduler at 16 warps an SM.
+// Measured on B200 against those: one build of (H2O)_32 / cc-pVDZ, (ps|ss) 18.7 ->
+// 13.7 ms, (ss|ss) 10.3 -> 6.6 ms, (ps|ps) 11.6 -> 8.6 ms, (ds|ds) 1.10 -> 0.71 ms, (dp|ps)
+// 4.1 -> 3.7 ms, (ds|pp) 2.3 -> 2.1 ms; C60H122 / 6-31G**, FP32 band, (ps|ss) 37.7 -> 30.3
+// ms, (dp|pp) 8.4 -> 7.3 ms, but (ds|pp) 5.8 -> 5.9 ms and (dp|ps) 10.7 -> 11.0 ms.  What
+// bounds it now is latency: 0.43 instructions a cycle and scheduler at 16 warps an SM.
 #pragma once
 #include "jk_common.cuh"
 
@@ -95,6 +96,13 @@ jk_warp(JKArgs A, JKTask T) {
     constexpr int GSZ = (LI + 1) * (LJ + 1) * (LK + 1) * (LL + 1);
     // roots one after another where unrolling them would make the code long
     constexpr int UNROLL_ROOTS = NR * NF <= 60 ? NR : 1;
+    // A large FP32 block is digested one fi at a time, so that few converted
+    // components (9 of the 54) are live beside it: 36 bytes of spill stores instead of 612 for
+    // (dp|ps); C60H122 / 6-31G**, FP32 band, (dp|pp) 8.2 -> 7.4 ms, (dp|ds) 5.2 -> 4.6
+    // ms.  In FP64, where nothing is converted, and for smaller blocks the other
+    // order is the better one: (dp|ps) 4.0 against 4.8 ms, (ds|ps) 4.3 against 4.8 ms
+    // of a build of (H2O)_32 / cc-pVDZ.
+    constexpr bool SLICES = sizeof(F) == 4 && NF >= LARGE_NF && NFJ * NKL <= 9;
     constexpr int S_KL = 0, S_IL = NKL, S_IK = NKL + NFI * NFL;   // slots of the carried sums
     extern __shared__ double s_sum[];
     const int lane = threadIdx.x & 31, half = lane >> 4, col = lane & 15;
@@ -265,90 +273,165 @@ jk_warp(JKArgs A, JKTask T) {
                     for (int n = 0; n < NIJ + NFJ * NFK; n++) v[n] = 0.;
                     // a lane that is screened out touches no density: it may hold anything
                     if (active) {
-                    // rows of the density: an element is one address step from its row
-                    const double *Di[NFI], *Dj[NFJ], *Dk[NFK];
+                        // rows of the density: an element is one address step from its row
+                        const double *Di[NFI], *Dj[NFJ], *Dk[NFK];
 #pragma unroll
-                    for (int n = 0; n < NFI; n++) Di[n] = D + (long long)(i0 + n) * nao;
+                        for (int n = 0; n < NFI; n++) Di[n] = D + (long long)(i0 + n) * nao;
 #pragma unroll
-                    for (int n = 0; n < NFJ; n++) Dj[n] = D + (long long)(j0 + n) * nao;
+                        for (int n = 0; n < NFJ; n++) Dj[n] = D + (long long)(j0 + n) * nao;
 #pragma unroll
-                    for (int n = 0; n < NFK; n++) Dk[n] = D + (long long)(k0 + n) * nao;
-                    if (A.vj != nullptr) {
+                        for (int n = 0; n < NFK; n++) Dk[n] = D + (long long)(k0 + n) * nao;
+                        if constexpr (SLICES) {
+                            double d_kl[NKL], d_jl[NFJ * NFL], d_jk[NFJ * NFK];
+                            double jkl[NKL], pjl[NFJ * NFL];
 #pragma unroll
-                        for (int kl = 0; kl < NKL; kl++) {
-                            const double d = __ldg(Dk[kl / NFL] + l0 + kl % NFL);
+                            for (int n = 0; n < NKL; n++) {
+                                d_kl[n] = A.vj != nullptr ? __ldg(Dk[n / NFL] + l0 + n % NFL) : 0.;
+                                jkl[n] = 0.;
+                            }
 #pragma unroll
-                            for (int ij = 0; ij < NIJ; ij++) v[ij] += (double)acc[ij * NKL + kl] * d;
+                            for (int n = 0; n < NFJ * NFL; n++) {
+                                d_jl[n] = A.vk != nullptr ? __ldg(Dj[n / NFL] + l0 + n % NFL) : 0.;
+                                pjl[n] = 0.;
+                            }
+#pragma unroll
+                            for (int n = 0; n < NFJ * NFK; n++)
+                                d_jk[n] = A.vk != nullptr ? __ldg(Dj[n / NFK] + k0 + n % NFK) : 0.;
+                            // one fi at a time
+#pragma unroll
+                            for (int fi = 0; fi < NFI; fi++) {
+                                double e[NFJ * NKL];
+#pragma unroll
+                                for (int n = 0; n < NFJ * NKL; n++) e[n] = (double)acc[fi * NFJ * NKL + n];
+                                if (A.vj != nullptr) {
+#pragma unroll
+                                    for (int fj = 0; fj < NFJ; fj++) {
+                                        const double d_ij = __ldg(Di[fi] + j0 + fj);
+#pragma unroll
+                                        for (int kl = 0; kl < NKL; kl++) {
+                                            v[fi * NFJ + fj] += e[fj * NKL + kl] * d_kl[kl];
+                                            jkl[kl] += e[fj * NKL + kl] * d_ij;
+                                        }
+                                    }
+                                }
+                                if (A.vk != nullptr) {
+#pragma unroll
+                                    for (int fl = 0; fl < NFL; fl++) {
+                                        const double d_il = __ldg(Di[fi] + l0 + fl);
+                                        double t = 0.;   // K_il
+#pragma unroll
+                                        for (int fj = 0; fj < NFJ; fj++)
+#pragma unroll
+                                            for (int fk = 0; fk < NFK; fk++) {
+                                                v[NIJ + fj * NFK + fk] += e[(fj * NFK + fk) * NFL + fl] * d_il;
+                                                t += e[(fj * NFK + fk) * NFL + fl] * d_jk[fj * NFK + fk];
+                                            }
+                                        sum_add(S_IL + fi * NFL + fl, t);
+                                    }
+#pragma unroll
+                                    for (int fk = 0; fk < NFK; fk++) {
+                                        const double d_ik = __ldg(Di[fi] + k0 + fk);
+                                        double t = 0.;   // K_ik
+#pragma unroll
+                                        for (int fj = 0; fj < NFJ; fj++)
+#pragma unroll
+                                            for (int fl = 0; fl < NFL; fl++) {
+                                                pjl[fj * NFL + fl] += e[(fj * NFK + fk) * NFL + fl] * d_ik;
+                                                t += e[(fj * NFK + fk) * NFL + fl] * d_jl[fj * NFL + fl];
+                                            }
+                                        sum_add(S_IK + fi * NFK + fk, t);
+                                    }
+                                }
+                            }
+                            if (A.vj != nullptr) {
+#pragma unroll
+                                for (int n = 0; n < NKL; n++) sum_add(S_KL + n, jkl[n]);
+                            }
+                            if (A.vk != nullptr) {
+                                // K_jl: one target per quartet
+#pragma unroll
+                                for (int n = 0; n < NFJ * NFL; n++)
+                                    atomicAdd(VK + (long long)(j0 + n / NFL) * kr + (long long)(l0 + n % NFL) * kc, pjl[n]);
+                            }
+                        } else {
+                            if (A.vj != nullptr) {
+#pragma unroll
+                                for (int kl = 0; kl < NKL; kl++) {
+                                    const double d = __ldg(Dk[kl / NFL] + l0 + kl % NFL);
+#pragma unroll
+                                    for (int ij = 0; ij < NIJ; ij++) v[ij] += (double)acc[ij * NKL + kl] * d;
+                                }
+                                // J_kl
+                                double d_ij[NIJ];
+#pragma unroll
+                                for (int n = 0; n < NIJ; n++) d_ij[n] = __ldg(Di[n / NFJ] + j0 + n % NFJ);
+#pragma unroll
+                                for (int kl = 0; kl < NKL; kl++) {
+                                    double t = 0.;
+#pragma unroll
+                                    for (int ij = 0; ij < NIJ; ij++) t += (double)acc[ij * NKL + kl] * d_ij[ij];
+                                    sum_add(S_KL + kl, t);
+                                }
+                            }
+                            if (A.vk != nullptr) {
+                                // K_jk
+#pragma unroll
+                                for (int fi = 0; fi < NFI; fi++)
+#pragma unroll
+                                    for (int fl = 0; fl < NFL; fl++) {
+                                        const double d = __ldg(Di[fi] + l0 + fl);
+#pragma unroll
+                                        for (int fj = 0; fj < NFJ; fj++)
+#pragma unroll
+                                            for (int fk = 0; fk < NFK; fk++)
+                                                v[NIJ + fj * NFK + fk] += ACC(fi, fj, fk, fl) * d;
+                                    }
+                                // K_jl: one target per quartet
+                                double pjl[NFJ * NFL];
+#pragma unroll
+                                for (int n = 0; n < NFJ * NFL; n++) pjl[n] = 0.;
+#pragma unroll
+                                for (int fi = 0; fi < NFI; fi++)
+#pragma unroll
+                                    for (int fk = 0; fk < NFK; fk++) {
+                                        const double d = __ldg(Di[fi] + k0 + fk);
+#pragma unroll
+                                        for (int fj = 0; fj < NFJ; fj++)
+#pragma unroll
+                                            for (int fl = 0; fl < NFL; fl++) pjl[fj * NFL + fl] += ACC(fi, fj, fk, fl) * d;
+                                    }
+#pragma unroll
+                                for (int n = 0; n < NFJ * NFL; n++)
+                                    atomicAdd(VK + (long long)(j0 + n / NFL) * kr + (long long)(l0 + n % NFL) * kc, pjl[n]);
+                                // K_ik
+                                double d_jl[NFJ * NFL];
+#pragma unroll
+                                for (int n = 0; n < NFJ * NFL; n++) d_jl[n] = __ldg(Dj[n / NFL] + l0 + n % NFL);
+#pragma unroll
+                                for (int fi = 0; fi < NFI; fi++)
+#pragma unroll
+                                    for (int fk = 0; fk < NFK; fk++) {
+                                        double t = 0.;
+#pragma unroll
+                                        for (int n = 0; n < NFJ * NFL; n++) t += ACC(fi, n / NFL, fk, n % NFL) * d_jl[n];
+                                        sum_add(S_IK + fi * NFK + fk, t);
+                                    }
+                                // K_il
+                                double d_jk[NFJ * NFK];
+#pragma unroll
+                                for (int n = 0; n < NFJ * NFK; n++) d_jk[n] = __ldg(Dj[n / NFK] + k0 + n % NFK);
+#pragma unroll
+                                for (int fi = 0; fi < NFI; fi++)
+#pragma unroll
+                                    for (int fl = 0; fl < NFL; fl++) {
+                                        double t = 0.;
+#pragma unroll
+                                        for (int n = 0; n < NFJ * NFK; n++) t += ACC(fi, n / NFK, n % NFK, fl) * d_jk[n];
+                                        sum_add(S_IL + fi * NFL + fl, t);
+                                    }
+                                }
                         }
-                        // J_kl
-                        double d_ij[NIJ];
-#pragma unroll
-                        for (int n = 0; n < NIJ; n++) d_ij[n] = __ldg(Di[n / NFJ] + j0 + n % NFJ);
-#pragma unroll
-                        for (int kl = 0; kl < NKL; kl++) {
-                            double t = 0.;
-#pragma unroll
-                            for (int ij = 0; ij < NIJ; ij++) t += (double)acc[ij * NKL + kl] * d_ij[ij];
-                            sum_add(S_KL + kl, t);
-                        }
-                    }
-                    if (A.vk != nullptr) {
-                        // K_jk
-#pragma unroll
-                        for (int fi = 0; fi < NFI; fi++)
-#pragma unroll
-                            for (int fl = 0; fl < NFL; fl++) {
-                                const double d = __ldg(Di[fi] + l0 + fl);
-#pragma unroll
-                                for (int fj = 0; fj < NFJ; fj++)
-#pragma unroll
-                                    for (int fk = 0; fk < NFK; fk++)
-                                        v[NIJ + fj * NFK + fk] += ACC(fi, fj, fk, fl) * d;
-                            }
-                        // K_jl: one target per quartet
-                        double pjl[NFJ * NFL];
-#pragma unroll
-                        for (int n = 0; n < NFJ * NFL; n++) pjl[n] = 0.;
-#pragma unroll
-                        for (int fi = 0; fi < NFI; fi++)
-#pragma unroll
-                            for (int fk = 0; fk < NFK; fk++) {
-                                const double d = __ldg(Di[fi] + k0 + fk);
-#pragma unroll
-                                for (int fj = 0; fj < NFJ; fj++)
-#pragma unroll
-                                    for (int fl = 0; fl < NFL; fl++) pjl[fj * NFL + fl] += ACC(fi, fj, fk, fl) * d;
-                            }
-#pragma unroll
-                        for (int n = 0; n < NFJ * NFL; n++)
-                            atomicAdd(VK + (long long)(j0 + n / NFL) * kr + (long long)(l0 + n % NFL) * kc, pjl[n]);
-                        // K_ik
-                        double d_jl[NFJ * NFL];
-#pragma unroll
-                        for (int n = 0; n < NFJ * NFL; n++) d_jl[n] = __ldg(Dj[n / NFL] + l0 + n % NFL);
-#pragma unroll
-                        for (int fi = 0; fi < NFI; fi++)
-#pragma unroll
-                            for (int fk = 0; fk < NFK; fk++) {
-                                double t = 0.;
-#pragma unroll
-                                for (int n = 0; n < NFJ * NFL; n++) t += ACC(fi, n / NFL, fk, n % NFL) * d_jl[n];
-                                sum_add(S_IK + fi * NFK + fk, t);
-                            }
-                        // K_il
-                        double d_jk[NFJ * NFK];
-#pragma unroll
-                        for (int n = 0; n < NFJ * NFK; n++) d_jk[n] = __ldg(Dj[n / NFK] + k0 + n % NFK);
-#pragma unroll
-                        for (int fi = 0; fi < NFI; fi++)
-#pragma unroll
-                            for (int fl = 0; fl < NFL; fl++) {
-                                double t = 0.;
-#pragma unroll
-                                for (int n = 0; n < NFJ * NFK; n++) t += ACC(fi, n / NFK, n % NFK, fl) * d_jk[n];
-                                sum_add(S_IL + fi * NFL + fl, t);
-                            }
-                        if (!ket_uni) {
+                        if (A.vk != nullptr && !ket_uni) {
                             // no shell k shared by the lanes: K_jk one by one
 #pragma unroll
                             for (int n = 0; n < NFJ * NFK; n++) {
@@ -356,7 +439,6 @@ jk_warp(JKArgs A, JKTask T) {
                                 v[NIJ + n] = 0.;
                             }
                         }
-                    }
                     }
                     half_warp_sum(v, lane, [&](int n, double y) {
                         double *dst = n < NIJ ? VJ + (size_t)(i0 + n / NFJ) * nao + j0 + n % NFJ
@@ -446,36 +528,53 @@ static int launch_warp_f(const JKArgs &args, const JKTask &task, cudaStream_t st
     return 0;
 }
 
-template <int LI, int LJ, int LK, int LL, int CK>
-static int launch_warp(const JKArgs &args, const JKTask &task, int fp32, cudaStream_t stream) {
+template <int LI, int LJ, int LK, int LL, int CK, typename F>
+static int launch_warp_t(const JKArgs &args, const JKTask &task, cudaStream_t stream) {
     JKTask t = task;
     t.ntiles = task_tiles(task);
     if (t.ntiles == 0) return 0;
     if (t.nsm <= 0 && (t.nsm = device_sms()) <= 0) return 1;
     if (t.ntiles_dev == nullptr) t.split = warp_split(t.ntiles, t.nsm);
     bqc_count_launch(cdiv(ncart(LK), CK) - 1);   // the dispatcher counted one
-    if (fp32) return launch_warp_f<LI, LJ, LK, LL, float, 0, CK>(args, t, stream);
-    return launch_warp_f<LI, LJ, LK, LL, double, 0, CK>(args, t, stream);
+    return launch_warp_f<LI, LJ, LK, LL, F, 0, CK>(args, t, stream);
+}
+
+template <int LI, int LJ, int LK, int LL, int CK>
+static int launch_warp(const JKArgs &args, const JKTask &task, int fp32, cudaStream_t stream) {
+    if (fp32) return launch_warp_t<LI, LJ, LK, LL, CK, float>(args, task, stream);
+    return launch_warp_t<LI, LJ, LK, LL, CK, double>(args, task, stream);
 }
 
 // A class of at most SMALL_NF components, in one of its two orientations.  The
 // lanes hold the ket pairs and carry J_kl, K_il and K_ik over the bra pairs:
-// the orientation that carries fewer sums.  From LARGE_NF components on it is the
-// one with fewer sums over the half warp, whose vector is live with the block:
-// one build of (H2O)_32 / cc-pVDZ, (dp|ps) with 9 of them 3.6 ms, with 27 3.9 ms,
-// (ds|pp) 2.2 and 2.4 ms.  Below, the carried sums cost more: (pp|ss) 5.1 ms
-// with 4 of them and 15 carried, 4.6 ms with 12 and 7, (pp|ps) 6.1 and 5.6 ms.
-template <int L1, int L2, int L3, int L4>
-static int launch_small(const JKArgs &args, const JKTask &task, int fp32, cudaStream_t stream) {
+// the orientation that carries fewer sums.  From LARGE_NF components on the
+// registers decide.  FP64: the one with fewer sums over the half warp, whose
+// vector is live with the block: one build of (H2O)_32 / cc-pVDZ, (dp|ps) with 9 of
+// them 3.6 ms, with 27 3.9 ms, (ds|pp) 2.2 and 2.4 ms.  Below, the carried sums
+// cost more: (pp|ss) 5.1 ms with 4 of them and 15 carried, 4.6 ms with 12 and 7,
+// (pp|ps) 6.1 and 5.6 ms.  FP32: the one with the smaller slices (jk_warp), 9
+// components against 18: C60H122 / 6-31G**, FP32 band, with the whole block and with
+// slices, (dp|ps) 12.1 -> 11.0 ms, (ds|pp) 6.6 -> 5.9 ms.
+template <int L1, int L2, int L3, int L4, typename F>
+static int launch_small_t(const JKArgs &args, const JKTask &task, cudaStream_t stream) {
     using C = WarpCfg<L1, L2, L3, L4, ncart(L3)>;
     using S = WarpCfg<L3, L4, L1, L2, ncart(L1)>;
-    if constexpr (C::NF < LARGE_NF ? S::PERS < C::PERS : S::RED < C::RED) {
+    constexpr bool swap = C::NF < LARGE_NF      ? S::PERS < C::PERS
+                          : sizeof(F) == 8      ? S::RED < C::RED
+                                                : S::NFI > C::NFI;
+    if constexpr (swap) {
         JKTask sw = jk_swap_task(task);
         sw.k_transposed = !sw.k_transposed;
-        return launch_warp<L3, L4, L1, L2, ncart(L1)>(jk_args_swap_eri(args), sw, fp32, stream);
+        return launch_warp_t<L3, L4, L1, L2, ncart(L1), F>(jk_args_swap_eri(args), sw, stream);
     } else {
-        return launch_warp<L1, L2, L3, L4, ncart(L3)>(args, task, fp32, stream);
+        return launch_warp_t<L1, L2, L3, L4, ncart(L3), F>(args, task, stream);
     }
+}
+
+template <int L1, int L2, int L3, int L4>
+static int launch_small(const JKArgs &args, const JKTask &task, int fp32, cudaStream_t stream) {
+    if (fp32) return launch_small_t<L1, L2, L3, L4, float>(args, task, stream);
+    return launch_small_t<L1, L2, L3, L4, double>(args, task, stream);
 }
 
 }  // namespace bqc
