@@ -1,5 +1,6 @@
 """The Rys polynomials (csrc/rys_poly.inc), both layouts, evaluated as the
-kernels do, against 60-digit golden nodes and weights."""
+kernels do below XMAX, against 60-digit golden nodes and weights (on the device,
+and on both sides of XMAX: test_gpu_rys.py)."""
 import json
 import os
 import re
