@@ -238,6 +238,10 @@ static int smem_attr(int bytes) {
 // cudaGetLastError().
 static inline void launch_at(void (*kernel)(JKArgs, JKTask), int grid, int block, size_t smem, cudaStream_t stream,
                              const JKArgs &args, const JKTask &task) {
+    if (task.ntiles_dev == nullptr || task.priority == 0) {
+        kernel<<<grid, block, smem, stream>>>(args, task);
+        return;
+    }
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributePriority;
     attr.val.priority = task.priority;
@@ -247,7 +251,7 @@ static inline void launch_at(void (*kernel)(JKArgs, JKTask), int grid, int block
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &attr;
-    cfg.numAttrs = task.ntiles_dev != nullptr && task.priority != 0;
+    cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, args, task);
 }
 
