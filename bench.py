@@ -275,11 +275,11 @@ def cpu_oracle_scf(threads):
                               threads, cycles))
 
 
-# DRAM bytes per launch of the J/K kernels (dram__bytes_read.sum +
-# dram__bytes_write.sum of one ncu --set full capture of one launch of the
-# class at (H2O)_64 / cc-pVTZ shape on the jk.py density), by class
-TRAFFIC = {'(ps|ss)': 72824320 + 38084352, '(dp|ps)': 300668672 + 132837376,
-           '(fp|dp)': 570294016 + 3547033000}
+# DRAM bytes of the longest launch of a class (dram__bytes_read.sum +
+# dram__bytes_write.sum, ncu, one pass) at (H2O)_64 / cc-pVTZ shape on the jk.py
+# density, by class
+TRAFFIC = {'(dp|ps)': 681786624 + 319410688, '(dp|ds)': 526273792 + 257069312,
+           '(ds|ps)': 514902016 + 226747136}
 
 
 def main():
